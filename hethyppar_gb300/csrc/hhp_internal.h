@@ -99,6 +99,7 @@ struct PlanDev {
     long long *slice_ptr = nullptr;   // n_slices + 1
     int *pos_row = nullptr;           // n_slices * H (original row, -1 = padding)
     int *pos_len = nullptr;           // n_slices * H
+    unsigned char *mask8 = nullptr;   // uniform diagonals, K = 5 or 7: pos_len's masks, a byte per row
     int *warp_ptr = nullptr;          // n_warps + 1
     int *warp_units = nullptr;        // unit ids (slice s < n_slices, else chunk n_slices + c)
     int4 *unit_rec = nullptr;         // per entry of warp_units: {unit, slice steps, slice start

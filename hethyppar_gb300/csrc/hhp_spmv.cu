@@ -139,6 +139,9 @@ struct SellArgs {
     int m, n_slices, n_chunks, n_long;
     bool has_perm;
     int doff[kMaxDiag];  // uniform-diagonal plans: the diagonals' offsets (pos_len then holds row masks)
+    const unsigned char *mask8;  // the same masks in a byte per row (plans of 5 or 7 diagonals)
+    int n;
+    bool x_vec;          // x starts on a 16-byte boundary
 };
 
 __device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
@@ -429,6 +432,41 @@ __device__ __forceinline__ void do_chunk(const SellArgs<VT> &a, int c, int lane)
     }
 }
 
+// The CTA's partial record of the epilogue's dot products.
+template <typename VT, int EP>
+__device__ __forceinline__ void cta_partials(const SellArgs<VT> &a, double d0, double d1, double d2, double *red,
+                                             int lane, int warp, int nw) {
+    if (EP == EP_DOT3) {
+        // records of 4: (d0, d1, d2, 0); each warp's transposed butterfly leaves quantity q in
+        // lanes [8q, 8q + 8), warp 0 adds the warps' results within each group of 8 lanes
+        const double dv[4] = {d0, d1, d2, 0.0};
+        const double r = warp_reduce<4>(dv, lane);
+        if ((lane & 7) == 0) red[lane + warp] = r;  // red[8q + warp], nw <= 8
+        __syncthreads();
+        if (warp == 0) {
+            double s = (lane < 24 && (lane & 7) < nw) ? red[lane] : 0.0;
+#pragma unroll
+            for (int o = 4; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if ((lane & 7) == 0) a.cta_part[4 * blockIdx.x + (lane >> 3)] = s;
+        }
+    } else if (EP != EP_AXPBY && EP != EP_Y) {
+        // per-CTA partial: each warp folds its lanes' (d0, d1) with a transposed butterfly
+        // (5 FP64 adds for both sums), warp 0 adds the warps' results; fixed order throughout
+        warp_sum2(d0, d1, lane);
+        if (lane == 0) red[warp] = d0;
+        if (lane == 16) red[8 + warp] = d1;
+        __syncthreads();
+        if (warp == 0) {
+            // lanes 0-7 take the warps' d0 sums, lanes 8-15 their d1 sums (nw <= 8 warps)
+            double s = (lane < 16 && (lane & 7) < nw) ? red[lane] : 0.0;
+#pragma unroll
+            for (int o = 4; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) a.cta_part[2 * blockIdx.x] = s;
+            if (lane == 8) a.cta_part[2 * blockIdx.x + 1] = s;
+        }
+    }
+}
+
 // Resident CTAs of 256 threads that the register need of R*U words in flight per lane allows.
 template <int R, int U>
 struct MinCtas {
@@ -471,34 +509,120 @@ __global__ void __launch_bounds__(256, MinCtasFor<VT, R, U, UNI>::value) k_spmv(
             do_chunk<VT, EP>(a, u - a.n_slices, lane);
         }
     }
-    if (EP == EP_DOT3) {
-        // records of 4: (d0, d1, d2, 0); each warp's transposed butterfly leaves quantity q in
-        // lanes [8q, 8q + 8), warp 0 adds the warps' results within each group of 8 lanes
-        const double dv[4] = {d0, d1, d2, 0.0};
-        const double r = warp_reduce<4>(dv, lane);
-        if ((lane & 7) == 0) red[lane + warp] = r;  // red[8q + warp], nw <= 8
-        __syncthreads();
-        if (warp == 0) {
-            double s = (lane < 24 && (lane & 7) < nw) ? red[lane] : 0.0;
-#pragma unroll
-            for (int o = 4; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if ((lane & 7) == 0) a.cta_part[4 * blockIdx.x + (lane >> 3)] = s;
+    cta_partials<VT, EP>(a, d0, d1, d2, red, lane, warp, nw);
+}
+
+// A lane's N consecutive entries x[i .. i + N), i = row + off with row a multiple of N: one vector load
+// when off is a multiple of N too (the same in every lane) and x is aligned (vec).
+template <typename VT, int N>
+__device__ __forceinline__ void load_run(VT (&o)[N], const VT *x, int i, int off, bool vec) {
+    if constexpr (N == 2) {
+        if (vec && (off & 1) == 0) {
+            const typename Vec<VT, 2>::V v = __ldg(reinterpret_cast<const typename Vec<VT, 2>::V *>(x + i));
+            o[0] = v.x;
+            o[1] = v.y;
+            return;
         }
-    } else if (EP != EP_AXPBY && EP != EP_Y) {
-        // per-CTA partial: each warp folds its lanes' (d0, d1) with a transposed butterfly
-        // (5 FP64 adds for both sums), warp 0 adds the warps' results; fixed order throughout
-        warp_sum2(d0, d1, lane);
-        if (lane == 0) red[warp] = d0;
-        if (lane == 16) red[8 + warp] = d1;
-        __syncthreads();
-        if (warp == 0) {
-            // lanes 0-7 take the warps' d0 sums, lanes 8-15 their d1 sums (nw <= 8 warps)
-            double s = (lane < 16 && (lane & 7) < nw) ? red[lane] : 0.0;
+    }
 #pragma unroll
-            for (int o = 4; o >= 1; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) a.cta_part[2 * blockIdx.x] = s;
-            if (lane == 8) a.cta_part[2 * blockIdx.x + 1] = s;
+    for (int t = 0; t < N; ++t) o[t] = __ldg(x + i + t);
+}
+
+// Uniform diagonals, K = 5 or 7 of them (2D and 3D stencils). The general kernel reads such a slice in
+// dependent rounds (work record, masks, a group of values and gathers, the last K mod U steps one by
+// one); here nothing waits for anything but the multiply-adds:
+//  * every unit costs the same, so a warp's units are gw, gw + W, ... (what the plan's dealing
+//    gives) and a slice starts at u K H: no work list;
+//  * a slice whose diagonals all stay inside x reads them without knowing its masks, which only
+//    select multiply-adds (a byte per row instead of the plan's four);
+//  * all K values and entries of x are requested at once. A lane's R rows take two passes of R/2, so
+//    that 2 K R/2 words fit the registers of the occupancy that HBM latency needs (32 warps per SM
+//    FP32, 40 FP64); the second pass finds its half of every sector of the value stream in L1. One
+//    pass at that occupancy spills, and with fewer warps it is slower (FP32, 160^3: 37 us).
+// Lanes own the same rows and units as in the general kernel, so the dot products' partial sums are
+// the same too, bit for bit. 160^3 7-point: FP32 32.8 -> 28.4 us (the mixed solve 119.8 -> 108.7 us
+// an iteration), FP64 60.2 -> 58.5 us; 256^2 5-point FP64 6.2 -> 4.2 us (23.0 -> 21.7 us a solve iteration).
+template <typename VT, int R, int K, int EP, int CTAS>
+__global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ SellArgs<VT> a) {
+    constexpr int H = 32 * R, N = R / 2;  // N rows per lane and pass
+    using VN = typename Vec<VT, N>::V;
+    using VV = typename Vec<VT, R>::V;
+    constexpr bool W1 = EP == EP_DOT1 || EP == EP_DOT2 || EP == EP_DOT3 || EP == EP_RESID;
+    __shared__ double red[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int gw = blockIdx.x * nw + warp, W = gridDim.x * nw;
+    const int err = __ldcg(a.err), gate = a.gate ? __ldcg(a.gate) : 1, stop = a.stop ? __ldcg(a.stop) : 0;
+    const bool skip = err != DEV_OK || gate == 0 || stop != 0;
+    double d0 = 0.0, d1 = 0.0, d2 = 0.0;
+    for (int u = gw; u < a.n_slices; u += W) {
+        const int q0 = u * H + lane * R;
+        const VT *vp = static_cast<const VT *>(a.sval) + static_cast<size_t>(u) * (K * H) + lane * R;
+        unsigned mw;
+        if constexpr (R == 4) mw = __ldg(reinterpret_cast<const unsigned *>(a.mask8 + q0));
+        else mw = __ldg(reinterpret_cast<const unsigned short *>(a.mask8 + q0));
+        // every diagonal of every row of the slice lies inside x
+        const bool safe = u * H + a.doff[0] >= 0 && u * H + H + a.doff[K - 1] <= a.n;
+        VT acc[R];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            VN v[K];
+            VT xv[K][N];
+#pragma unroll
+            for (int k = 0; k < K; ++k) v[k] = __ldg(reinterpret_cast<const VN *>(vp + k * H + N * h));
+            if (safe) {
+#pragma unroll
+                for (int k = 0; k < K; ++k) load_run<VT, N>(xv[k], a.x, q0 + N * h + a.doff[k], a.doff[k], a.x_vec);
+            } else {
+#pragma unroll
+                for (int k = 0; k < K; ++k)
+#pragma unroll
+                    for (int t = 0; t < N; ++t)
+                        xv[k][t] = ((mw >> (8 * (N * h + t) + k)) & 1) ? __ldg(a.x + q0 + N * h + t + a.doff[k]) : VT(0);
+            }
+            if (h == 0 && u == gw && skip) return;  // before any store (uniform across the grid)
+#pragma unroll
+            for (int t = 0; t < N; ++t) acc[N * h + t] = VT(0);
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+                for (int t = 0; t < N; ++t)
+                    if ((mw >> (8 * (N * h + t) + k)) & 1)
+                        acc[N * h + t] = vfma(comp<VN, VT>(v[k], t), xv[k][t], acc[N * h + t]);
         }
+        VT w1v[R], w2v[R];
+        VV z1 = VV(), z2 = VV();
+        if (W1 && q0 < a.m) z1 = __ldg(reinterpret_cast<const VV *>(a.w1 + q0));
+        if (EP == EP_DOT3 && q0 < a.m) z2 = __ldg(reinterpret_cast<const VV *>(a.w2 + q0));
+#pragma unroll
+        for (int t = 0; t < R; ++t) {
+            w1v[t] = comp<VV, VT>(z1, t);
+            w2v[t] = comp<VV, VT>(z2, t);
+        }
+        VT e0 = VT(0), e1 = VT(0), e2 = VT(0);
+#pragma unroll
+        for (int t = 0; t < R; ++t)
+            if (q0 + t < a.m) row_epilogue<VT, EP>(a, q0 + t, acc[t], e0, e1, e2, w1v[t], w2v[t]);
+        if (EP != EP_AXPBY && EP != EP_Y) {
+            d0 += widen(e0);
+            d1 += widen(e1);
+        }
+        if (EP == EP_DOT3) d2 += widen(e2);
+    }
+    if (skip) return;
+    cta_partials<VT, EP>(a, d0, d1, d2, red, lane, warp, nw);
+}
+
+template <typename VT, int R, int K, int CTAS>
+cudaError_t launch_uni(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
+    const dim3 grid(p.ctas), block(p.warps_per_cta * 32);
+    switch (ep) {
+        case EP_DOT1: return launch_k(k_spmv_uni<VT, R, K, EP_DOT1, CTAS>, grid, block, 0, s, a);
+        case EP_DOT2: return launch_k(k_spmv_uni<VT, R, K, EP_DOT2, CTAS>, grid, block, 0, s, a);
+        case EP_DOT3: return launch_k(k_spmv_uni<VT, R, K, EP_DOT3, CTAS>, grid, block, 0, s, a);
+        case EP_RESID: return launch_k(k_spmv_uni<VT, R, K, EP_RESID, CTAS>, grid, block, 0, s, a);
+        default:
+            if (!a.scale && !a.accum) return launch_k(k_spmv_uni<VT, R, K, EP_Y, CTAS>, grid, block, 0, s, a);
+            return launch_k(k_spmv_uni<VT, R, K, EP_AXPBY, CTAS>, grid, block, 0, s, a);
     }
 }
 
@@ -532,6 +656,12 @@ cudaError_t launch_ru(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaSt
 template <typename VT>
 cudaError_t launch_ep(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
     const bool u2 = p.unroll == 2;
+    if (p.mask8) {  // 5 or 7 uniform diagonals in the default row layout
+        if constexpr (std::is_same<VT, double>::value)
+            return p.K == 5 ? launch_uni<VT, 2, 5, 5>(ep, p, a, s) : launch_uni<VT, 2, 7, 5>(ep, p, a, s);
+        else
+            return p.K == 5 ? launch_uni<VT, 4, 5, 4>(ep, p, a, s) : launch_uni<VT, 4, 7, 4>(ep, p, a, s);
+    }
     if constexpr (std::is_same<VT, double>::value) {
         if (p.rpl == 1) return u2 ? launch_ru<VT, 1, 2>(ep, p, a, s) : launch_ru<VT, 1, 4>(ep, p, a, s);
         return u2 ? launch_ru<VT, 2, 2>(ep, p, a, s) : launch_ru<VT, 2, 4>(ep, p, a, s);
@@ -696,6 +826,13 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
     p.release();
     p.uni = uni;
     p.K = K;
+    // the unrolled stencil kernel's masks (k_spmv_uni; other diagonal counts run the general kernel)
+    if (uni && (K == 5 || K == 7) && R == (std::is_same<VT, double>::value ? 2 : 4)) {
+        std::vector<unsigned char> m8(h.pos_len.size());
+        for (size_t q = 0; q < m8.size(); ++q) m8[q] = static_cast<unsigned char>(h.pos_len[q]);
+        HHP_TRY(upload(&p.mask8, m8, ctx->stream, 4));
+        HHP_CUDA(cudaStreamSynchronize(ctx->stream));
+    }
     for (int k = 0; k < kMaxDiag; ++k) p.doff[k] = doff[k];
     p.rpl = R;
     p.unroll = U;
@@ -834,6 +971,9 @@ SellArgs<VT> make_args(hhp_mat *A, const PlanDev &p, const VT *csr_val, const VT
     a.n_long = p.n_long;
     a.has_perm = p.has_perm;
     for (int k = 0; k < kMaxDiag; ++k) a.doff[k] = p.doff[k];
+    a.mask8 = p.mask8;
+    a.n = A->n;
+    a.x_vec = reinterpret_cast<uintptr_t>(x) % 16 == 0;
     return a;
 }
 
@@ -843,6 +983,7 @@ void PlanDev::release() {
     cudaFree(slice_ptr);
     cudaFree(pos_row);
     cudaFree(pos_len);
+    cudaFree(mask8);
     cudaFree(warp_ptr);
     cudaFree(warp_units);
     cudaFree(unit_rec);
