@@ -19,34 +19,40 @@ from ._lib import ITER_CB, HHPError, SolveInfo, SolveOpts, check, lib
 PRECISIONS = {"fp64": 0, "mixed": 1}
 
 
-def _ptr(a) -> ctypes.c_void_p:
+def _ptr(a):
     if a is None:
-        return ctypes.c_void_p(None)
+        return None
     if hasattr(a, "data_ptr"):
-        return ctypes.c_void_p(a.data_ptr())
+        return a.data_ptr()
     return a.ctypes.data_as(ctypes.c_void_p)
 
 
 class _Ordered:
     """Orders a library call on device tensors with torch's current stream: the context's stream
     waits for the work torch has queued (the inputs), and torch's stream waits for the call's work
-    (the outputs). Event waits on the device, no host synchronisation."""
+    (the outputs). Event waits on the device, no host synchronisation. The events are the context's
+    own, recorded by the library (hhp_ctx_wait_for / hhp_ctx_release_to): with torch's stream and
+    event objects, made anew for each call, the ordering took 16 of a small call's 19 us."""
+
+    __slots__ = ("ctx", "stream")
 
     def __init__(self, ctx, *tensors):
-        self.on = any(hasattr(t, "data_ptr") for t in tensors)
         self.ctx = ctx
+        self.stream = None
+        for t in tensors:
+            if hasattr(t, "data_ptr"):
+                import torch
+                self.stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+                break
 
     def __enter__(self):
-        if self.on:
-            import torch
-            self.ext = torch.cuda.ExternalStream(self.ctx.stream)
-            self.cur = torch.cuda.current_stream()
-            self.ext.wait_stream(self.cur)
+        if self.stream is not None:
+            check(lib().hhp_ctx_wait_for(self.ctx.handle, self.stream), "hhp_ctx_wait_for")
         return self
 
     def __exit__(self, *exc):
-        if self.on:
-            self.cur.wait_stream(self.ext)
+        if self.stream is not None:
+            check(lib().hhp_ctx_release_to(self.ctx.handle, self.stream), "hhp_ctx_release_to")
         return False
 
 

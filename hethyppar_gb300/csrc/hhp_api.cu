@@ -208,6 +208,7 @@ hhp_status hhp_ctx_create(int device, hhp_ctx **out) {
     c->smem_optin = prop.sharedMemPerBlockOptin;
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c->ev0) != cudaSuccess || cudaEventCreate(&c->ev1) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaMalloc(&c->dev_err, sizeof(int)) != cudaSuccess ||
         cudaMemsetAsync(c->dev_err, 0, sizeof(int), c->stream) != cudaSuccess ||
         cudaStreamSynchronize(c->stream) != cudaSuccess) {
@@ -227,6 +228,7 @@ void hhp_ctx_destroy(hhp_ctx *c) {
     if (c->dev_err) cudaFree(c->dev_err);
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
+    if (c->ev_join) cudaEventDestroy(c->ev_join);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
 }
@@ -236,6 +238,22 @@ void *hhp_ctx_stream(hhp_ctx *c) { return c ? static_cast<void *>(c->stream) : n
 hhp_status hhp_ctx_sync(hhp_ctx *c) {
     if (!c) return HHP_ERR_ARG;
     HHP_CUDA(cudaStreamSynchronize(c->stream));
+    return HHP_OK;
+}
+
+hhp_status hhp_ctx_wait_for(hhp_ctx *c, void *stream) {
+    if (!c) return HHP_ERR_ARG;
+    std::lock_guard<std::mutex> lock(c->join_mu);
+    HHP_CUDA(cudaEventRecord(c->ev_join, static_cast<cudaStream_t>(stream)));
+    HHP_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+    return HHP_OK;
+}
+
+hhp_status hhp_ctx_release_to(hhp_ctx *c, void *stream) {
+    if (!c) return HHP_ERR_ARG;
+    std::lock_guard<std::mutex> lock(c->join_mu);
+    HHP_CUDA(cudaEventRecord(c->ev_join, c->stream));
+    HHP_CUDA(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), c->ev_join, 0));
     return HHP_OK;
 }
 

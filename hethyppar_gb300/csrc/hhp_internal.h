@@ -5,6 +5,7 @@
 
 #include <cstdint>
 #include <exception>
+#include <mutex>
 #include <new>
 #include <cstdio>
 #include <string>
@@ -135,6 +136,8 @@ struct hhp_ctx {
     size_t smem_optin = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t ev_join = nullptr;    // orders this stream and a caller's (no timing)
+    std::mutex join_mu;               // one record and its wait at a time
     int *dev_err = nullptr;           // device error word (hhp::DEV_*), zeroed
     long long kernel_launches = 0;
     double *dot_part = nullptr;       // BLAS-1 dot: block partials (allocated on first use)

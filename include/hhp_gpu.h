@@ -130,6 +130,11 @@ void hhp_ctx_destroy(hhp_ctx *ctx);
 /* The context's cudaStream_t, as an opaque pointer. */
 void *hhp_ctx_stream(hhp_ctx *ctx);
 hhp_status hhp_ctx_sync(hhp_ctx *ctx);
+/* Order the context's stream after the work queued so far on `stream` (a cudaStream_t), and `stream`
+ * after the context's queued work, by an event on the device; the host does not wait. Callers with
+ * their own streams put them around a `_dev` call. */
+hhp_status hhp_ctx_wait_for(hhp_ctx *ctx, void *stream);
+hhp_status hhp_ctx_release_to(hhp_ctx *ctx, void *stream);
 /* Number of kernels this context has launched (graph launches count their kernel nodes). */
 long long hhp_ctx_kernel_launches(const hhp_ctx *ctx);
 /* No counterpart in the reference: the device's FP64 fused multiply-add throughput (lane FMAs per
