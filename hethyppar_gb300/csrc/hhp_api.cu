@@ -616,7 +616,7 @@ hhp_status hhp_ilu0_apply_dev(hhp_ctx *ctx, hhp_mat *A, const double *r_dev, dou
         return HHP_ERR_ARG;
     }
     HHP_TRY(ensure_ilu(A));
-    HHP_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream));
+    if (ilu_waits(A)) HHP_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), ctx->stream));
     return launch_ilu_apply(A, ctx->stream, r_dev, z_dev, nullptr);
     HHP_API_END
 }

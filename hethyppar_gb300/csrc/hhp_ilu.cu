@@ -45,12 +45,16 @@ namespace hhp {
 constexpr int kIluLong = 64;           // triangle entries above which a row is summed by a warp
 constexpr int kIluBig = 2048;          // ... and above which by a whole block
 constexpr int kIluThreads = 1024;      // threads per block of the cooperative kernels (32 warps)
+constexpr int kIluSegs = 8;            // runs of equally wide level-1 slices that k_ilu_half takes
 constexpr unsigned kBarrierSpins = 1u << 22;  // bounded wait (x ~64 ns sleeps: well under a second)
 
 struct IluTri {
     int n_levels = 0, n_slices = 0, n_long = 0, n_big = 0;
     int head_slice = 0, head_long = 0, head_big = 0;  // lev_*[min(2, n_levels)], kept on the host
     int lev1_slice = 0;                               // lev_slice[1]: the first level-1 slice
+    int n_seg = 0;                                    // level 1's runs of equally wide slices (0: too many)
+    int seg_slice[kIluSegs + 1] = {}, seg_width[kIluSegs] = {};
+    long long seg_slot[kIluSegs] = {};
     long long slots = 0;
     int *lev_slice = nullptr;        // n_levels + 1: the slices of each level
     int *lev_long = nullptr;         // n_levels + 1: the long rows of each level
@@ -59,6 +63,8 @@ struct IluTri {
     int *slice_row = nullptr;        // n_slices * 32 rows (-1: padding)
     int *slice_len = nullptr;        // n_slices * 32 entry counts
     int *scol = nullptr;             // slots: columns
+    unsigned short *scol16 = nullptr;  // slots: column - row - bias, where that fits (k_ilu_half)
+    int bias = 0;
     double *sval = nullptr;          // slots: factor values (filled after the factorization)
     int *long_row = nullptr;         // n_long
     int *big_row = nullptr;          // n_big
@@ -71,6 +77,7 @@ struct IluTri {
         cudaFree(slice_row);
         cudaFree(slice_len);
         cudaFree(scol);
+        cudaFree(scol16);
         cudaFree(sval);
         cudaFree(long_row);
         *this = IluTri();
@@ -102,6 +109,11 @@ struct IluDev {
 };
 
 namespace {
+
+// Both passes of a two-colour application fit k_ilu_half.
+bool ilu_halves(const IluDev &I) {
+    return I.two_colour && I.L.n_seg > 0 && I.U.n_seg > 0 && I.L.n_long + I.L.n_big + I.U.n_long + I.U.n_big == 0;
+}
 
 struct TriArgs {
     int n_levels;
@@ -365,6 +377,70 @@ __global__ void __launch_bounds__(kIluThreads, 1) k_ilu_tri(TriArgs t, const int
     }
 }
 
+
+// One pass of a two-colour application (see launch_ilu_apply) whose rows are all short: a warp per
+// slice, out_i = (in_i - sum v_k dep[c_k]) * (1 / u_ii) in ascending k. It is bound by the latency of
+// its dependent requests, so there are two rounds of them: the slots of a slice lie where the run of
+// equally wide slices that it belongs to says (arguments: no slice pointer is read), so the slots
+// and the row data are requested together, then the gathers, in_i and 1 / u_ii. One slice per warp
+// and 48 resident warps per SM measured best (an application on the 1024^2 5-point stencil, two
+// passes, back to back: two slices at 32 warps 24.0 us, 64 warps 30.6, 48 warps 23.5; k_ilu_tri,
+// whose slices take three dependent rounds, 30.8). COL16: columns as 16-bit distances from row +
+// bias, where all of the triangle's fit (10 bytes a slot instead of 12): 27.3 instead of 30.7 us from
+// HBM, 20.5 instead of 20.9 back to back; the ILU(0) solve 141.9 -> 124.7 us an iteration, on 256^2
+// (launch-bound) 50.2 -> 34.8.
+struct HalfArgs {
+    int n_seg, seg_slice[kIluSegs + 1], seg_width[kIluSegs];
+    long long seg_slot[kIluSegs];
+    const int *slice_row, *slice_len, *scol;
+    const unsigned short *scol16;
+    int bias;
+    const double *sval;
+};
+template <bool COL16>
+__global__ void __launch_bounds__(256, 6) k_ilu_half(const __grid_constant__ HalfArgs h, const double *__restrict__ dinv,
+                                                     const double *in, const double *dep, double *out, const int *stop,
+                                                     int *dev_err) {
+    const int lane = threadIdx.x & 31;
+    const int s = h.seg_slice[0] + static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    // inside the solve loop: nothing to do once it has ended or an error is recorded; a lone
+    // application starts from a clean error word instead (its passes wait for nothing)
+    const int run = stop ? __ldcg(stop) : ST_RUNNING, err = stop ? __ldcg(dev_err) : DEV_OK;
+    if (!stop && blockIdx.x == 0 && threadIdx.x == 0) *dev_err = DEV_OK;
+    if (s >= h.seg_slice[h.n_seg]) return;
+    const int row = __ldg(h.slice_row + 32 * s + lane), len = __ldg(h.slice_len + 32 * s + lane);
+    int width = h.seg_width[0];
+    long long q = h.seg_slot[0] + 32ll * width * (s - h.seg_slice[0]);
+    for (int g = 1; g < h.n_seg; ++g)
+        if (s >= h.seg_slice[g]) {
+            width = h.seg_width[g];
+            q = h.seg_slot[g] + 32ll * width * (s - h.seg_slice[g]);
+        }
+    q += lane;
+    double a = 0.0, d = 0.0;
+    for (int k = 0; k < width; k += 4) {
+        int c[4];
+        double v[4], z[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const bool on = k + j < width;
+            c[j] = !on ? 0 : COL16 ? static_cast<int>(__ldg(h.scol16 + q + 32 * (k + j))) : __ldg(h.scol + q + 32 * (k + j));
+            v[j] = on ? __ldg(h.sval + q + 32 * (k + j)) : 0.0;
+        }
+        if (k == 0) {
+            if (run != ST_RUNNING || err != DEV_OK) return;
+            a = row >= 0 ? in[row] : 0.0;
+            d = row >= 0 ? __ldg(dinv + row) : 0.0;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) z[j] = k + j < len ? dep[COL16 ? row + h.bias + c[j] : c[j]] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (k + j < len) a = fma(-v[j], z[j], a);
+    }
+    if (row >= 0) out[row] = a * d;
+}
+
 // Slot values and u_ii from the factor (sidx: the CSR position of every slot).
 __global__ void k_ilu_fill(const double *__restrict__ lu, const int *__restrict__ sidx, long long slots,
                            double *__restrict__ sval) {
@@ -462,6 +538,42 @@ hhp_status upload_tri(const TriHost &h, IluTri &d, int **sidx_dev, cudaStream_t 
     d.head_long = h.lev_long[head];
     d.head_big = h.lev_big[head];
     d.lev1_slice = h.n_levels >= 2 ? h.lev_slice[1] : 0;
+    // runs of equally wide slices on level 1 (its rows are sorted by length, so there are few)
+    for (int q = d.lev1_slice; h.n_levels == 2 && q < d.n_slices; ++q) {
+        const size_t sl = static_cast<size_t>(q);
+        const int width = static_cast<int>((h.slice_ptr[sl + 1] - h.slice_ptr[sl]) / 32);
+        if (d.n_seg == 0 || width != d.seg_width[d.n_seg - 1]) {
+            if (d.n_seg == kIluSegs) {
+                d.n_seg = 0;
+                break;
+            }
+            d.seg_slice[d.n_seg] = q;
+            d.seg_slot[d.n_seg] = h.slice_ptr[sl];
+            d.seg_width[d.n_seg++] = width;
+        }
+        d.seg_slice[d.n_seg] = q + 1;
+    }
+    if (d.n_seg > 0) {
+        // column - row over the slots' entries: a 16-bit range?
+        int lo = 0x7fffffff, hi = -0x7fffffff;
+        auto entries = [&](auto fn) {
+            for (int sl = 0; sl < d.n_slices; ++sl)
+                for (int j = 0; j < 32; ++j)
+                    for (int k = 0; k < h.slice_len[32 * static_cast<size_t>(sl) + static_cast<size_t>(j)]; ++k)
+                        fn(static_cast<size_t>(h.slice_ptr[static_cast<size_t>(sl)] + 32ll * k + j),
+                           h.slice_row[32 * static_cast<size_t>(sl) + static_cast<size_t>(j)]);
+        };
+        entries([&](size_t q, int row) {
+            lo = std::min(lo, h.scol[q] - row);
+            hi = std::max(hi, h.scol[q] - row);
+        });
+        if (lo <= hi && hi - lo <= 65535) {
+            d.bias = lo;
+            std::vector<unsigned short> c16(h.scol.size(), 0);
+            entries([&](size_t q, int row) { c16[q] = static_cast<unsigned short>(h.scol[q] - row - lo); });
+            HHP_TRY(upload(&d.scol16, c16, st));
+        }
+    }
     HHP_TRY(upload(&d.lev_slice, h.lev_slice, st));
     HHP_TRY(upload(&d.lev_long, h.lev_long, st));
     HHP_TRY(upload(&d.slice_ptr, h.slice_ptr, st));
@@ -733,6 +845,8 @@ hhp_status ensure_ilu(hhp_mat *A, int *levels) {
 
 long long ilu_generation(const hhp_mat *A) { return A->ilu ? A->ilu->gen : 0; }
 
+bool ilu_waits(const hhp_mat *A) { return A->ilu && !ilu_halves(*A->ilu); }
+
 void release_ilu(hhp_mat *A) {
     free_ilu(A->ilu);
     A->ilu = nullptr;
@@ -761,6 +875,28 @@ hhp_status launch_ilu_apply(hhp_mat *A, cudaStream_t st, const double *in, doubl
         // whose y is r itself: the backward pass reads r and the forward pass's results. Each
         // pass walks half the rows, y is not used, and every value is the one the two full
         // solves give, bit for bit (same sums, same order, the same multiplication by 1 / u_ii).
+        if (ilu_halves(*I)) {
+            auto pass = [&](const IluTri &t, const double *dep) {
+                HalfArgs h;
+                h.n_seg = t.n_seg;
+                std::copy(t.seg_slice, t.seg_slice + kIluSegs + 1, h.seg_slice);
+                std::copy(t.seg_width, t.seg_width + kIluSegs, h.seg_width);
+                std::copy(t.seg_slot, t.seg_slot + kIluSegs, h.seg_slot);
+                h.slice_row = t.slice_row;
+                h.slice_len = t.slice_len;
+                h.scol = t.scol;
+                h.scol16 = t.scol16;
+                h.bias = t.bias;
+                h.sval = t.sval;
+                const int n = t.seg_slice[t.n_seg] - t.seg_slice[0];
+                return launch_k(t.scol16 ? k_ilu_half<true> : k_ilu_half<false>, dim3((n + 7) / 8), dim3(256), 0, st, h,
+                                dinv, in, dep, out, stop, err);
+            };
+            HHP_CUDA(pass(I->L, in));
+            HHP_CUDA(pass(I->U, out));
+            A->ctx->kernel_launches += 2;
+            return HHP_OK;
+        }
         unsigned *b = I->bar, *bo = I->bar + 1;
         const double *x = in;
         double *y = out;

@@ -229,6 +229,9 @@ void release_ilu(hhp_mat *A);
 // Before hhp_mat_drop_csr frees A->col: factors that read their columns there take it over.
 void ilu_keep_col(hhp_mat *A);
 hhp_status launch_ilu_apply(hhp_mat *A, cudaStream_t st, const double *in, double *out, const int *stop);
+// The application's kernels check the context's error word (and may wait on a grid barrier); one that
+// does not clears the word itself when it is launched without `stop`.
+bool ilu_waits(const hhp_mat *A);
 hhp_status ilu_factors(hhp_mat *A, double *lu_host);
 // Identifies the current factorization (0: none); graphs that captured its arrays compare it.
 long long ilu_generation(const hhp_mat *A);
