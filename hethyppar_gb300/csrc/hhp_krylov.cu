@@ -62,6 +62,9 @@ constexpr size_t kCtlBytes = offsetof(DevScal, rho_prev);
 struct Solver {
     hhp_mat *A = nullptr;
     int n = 0, n_pad = 0, nblk = 0, nthr = 512;
+    // threads per block of the kernels without dot products (K_P, K_XRP and their mixed forms), per
+    // vector unit type; see update_threads
+    int nthr_u64 = 512, nthr_u32 = 512;
     // FP64 vectors (n_pad each)
     double *X = nullptr, *B = nullptr, *R = nullptr, *R0 = nullptr, *P = nullptr, *V = nullptr, *S = nullptr,
            *T = nullptr, *Y = nullptr;
@@ -1228,6 +1231,14 @@ T *dalloc(size_t n, hhp_status &st, cudaStream_t stream) {
 // The SpMV's partial records: one per CTA, then one per group of long rows.
 SpmvParts parts_of(const PlanDev &p) { return SpmvParts{p.cta_part, p.ctas, p.group_dot, p.n_groups}; }
 
+// A short vector has fewer units than 512-thread blocks have threads: its units then fill the first
+// blocks' warps and leave the other SMs' FP64 pipes idle. The kernels that form no dot product give
+// the same bits with any number of threads, so they take the smallest of 128, 256 and 512 (128: the
+// four warps that reduce the records) that covers the vector once.
+// 64^2 stencil 20.9 -> 19.7 us an iteration, 256^2 21.7 -> 20.7 (mixed 21.9 -> 20.7, classic 27.3 ->
+// 25.8); above 78k rows nothing changes.
+int update_threads(int nblk, int nu) { return nu <= nblk * 128 ? 128 : nu <= nblk * 256 ? 256 : 512; }
+
 hhp_status ensure_solver(hhp_mat *A, Solver **out, int maxit) {
     Solver *s = A->solver;
     if (!s) {
@@ -1237,6 +1248,8 @@ hhp_status ensure_solver(hhp_mat *A, Solver **out, int maxit) {
         s->n_pad = pad4(A->n);
         s->nblk = std::max(1, A->ctx->num_sms * tuning().vec_blocks_per_sm);
         s->unroll = std::max(1, std::min(tuning().unroll_iters, 16));
+        s->nthr_u64 = update_threads(s->nblk, s->n_pad / 2);
+        s->nthr_u32 = update_threads(s->nblk, s->n_pad / 4);
         hhp_status st = HHP_OK;
         const size_t np = static_cast<size_t>(s->n_pad);
         s->X = dalloc<double>(np, st, A->ctx->stream);
@@ -1406,7 +1419,7 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
     const int *stop = &sc->status;
     hhp_status st = HHP_OK;
     auto kp = [&](cudaStream_t q, cudaGraphConditionalHandle c, int first_in_body) -> hhp_status {
-        HHP_CUDA(launch_k(k_p<T>, dim3(s->nblk), dim3(s->nthr), 0, q, sc, P, V, R, nu, part_xr, part_s, s->nblk,
+        HHP_CUDA(launch_k(k_p<T>, dim3(s->nblk), dim3(fp32 ? s->nthr_u32 : s->nthr_u64), 0, q, sc, P, V, R, nu, part_xr, part_s, s->nblk,
                           s->hist, s->hist_cap, c, first_in_body, A->ctx->dev_err, 1,
                           static_cast<const int *>(nullptr)));
         return HHP_OK;
@@ -1441,7 +1454,7 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
                 }
                 st = launch_spmv64(A, s->s2, EP_DOT3, sv, Tv, S, 1.0, 0.0, nullptr, R0, stop);
                 if (st != HHP_OK) break;
-                if (launch_k(ilu ? k_xrp<double, true> : k_xrp<double, false>, dim3(s->nblk), dim3(s->nthr), 0,
+                if (launch_k(ilu ? k_xrp<double, true> : k_xrp<double, false>, dim3(s->nblk), dim3(s->nthr_u64), 0,
                              s->s2, sc, X, R, P, S, Tv, V, nu, parts_of(pl), part_s, s->nblk, s->hist,
                              s->hist_cap, cond, k == 0 ? 1 : 0, A->ctx->dev_err, 1, pv, sv) != cudaSuccess)
                     st = HHP_ERR_CUDA;
@@ -1467,7 +1480,7 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
             }
             st = launch_spmv32(A, s->s2, EP_DOT3, S, Tv, S, stop, R0);
             if (st != HHP_OK) break;
-            if (launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr), 0, s->s2, s->sc32, s->X, s->D32, s->R32, s->P32,
+            if (launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, s->s2, s->sc32, s->X, s->D32, s->R32, s->P32,
                          s->S32, s->T32, s->V32, nu4, parts_of(pl), part_s, s->nblk, s->hist, s->hist_cap, cond,
                          icond_body, k == 0 ? 1 : 0, A->ctx->dev_err, 1) != cudaSuccess) {
                 st = HHP_ERR_CUDA;
@@ -1545,7 +1558,7 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
         cudaGraphConditionalHandle icond;
         st = make_cond_if(s->s2, &icond);
         if (st != HHP_OK) break;
-        if (launch_k(k_p_ru, dim3(s->nblk), dim3(s->nthr), 0, s->s2, s->sc32, s->X, s->D32, s->P32, s->V32, s->R32,
+        if (launch_k(k_p_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, s->s2, s->sc32, s->X, s->D32, s->P32, s->V32, s->R32,
                      nu4, s->part_xr32, s->part_s32, s->nblk, s->hist, s->hist_cap, cond, icond, k == 0 ? 1 : 0,
                      A->ctx->dev_err, 1) != cudaSuccess) {
             st = HHP_ERR_CUDA;
@@ -1588,7 +1601,7 @@ hhp_status run_direct64(Solver *s, bool merged, bool ilu) {
     A->ctx->kernel_launches += 2;
     const PlanDev &pl = A->plan64;
     auto kp = [&](int first) -> hhp_status {
-        HHP_CUDA(launch_k(k_p<double>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc, s->P, s->V, s->R, nu, s->part_xr,
+        HHP_CUDA(launch_k(k_p<double>, dim3(s->nblk), dim3(s->nthr_u64), 0, st, s->sc, s->P, s->V, s->R, nu, s->part_xr,
                           s->part_s, s->nblk, s->hist, s->hist_cap, cudaGraphConditionalHandle(), first,
                           A->ctx->dev_err, 0, static_cast<const int *>(nullptr)));
         A->ctx->kernel_launches += 1;
@@ -1611,7 +1624,7 @@ hhp_status run_direct64(Solver *s, bool merged, bool ilu) {
                     sv = s->SH;
                 }
                 HHP_TRY(launch_spmv64(A, st, EP_DOT3, sv, s->T, s->S, 1.0, 0.0, nullptr, s->R0, stop));
-                HHP_CUDA(launch_k(ilu ? k_xrp<double, true> : k_xrp<double, false>, dim3(s->nblk), dim3(s->nthr), 0,
+                HHP_CUDA(launch_k(ilu ? k_xrp<double, true> : k_xrp<double, false>, dim3(s->nblk), dim3(s->nthr_u64), 0,
                                   st, s->sc, s->X, s->R, s->P, s->S, s->T, s->V, nu, parts_of(pl), s->part_s, s->nblk,
                                   s->hist, s->hist_cap, cudaGraphConditionalHandle(), k == 0 ? 1 : 0,
                                   A->ctx->dev_err, 0, pv, sv));
@@ -1773,7 +1786,7 @@ hhp_status run_direct_mix(Solver *s, bool merged) {
                       s->part_s32));
     nk += 2;
     auto kp = [&](int first, const int *gate) -> hhp_status {
-        HHP_CUDA(launch_k(k_p<float>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->P32, s->V32, s->R32, nu4,
+        HHP_CUDA(launch_k(k_p<float>, dim3(s->nblk), dim3(s->nthr_u32), 0, st, s->sc32, s->P32, s->V32, s->R32, nu4,
                           s->part_xr32, s->part_s32, s->nblk, s->hist, s->hist_cap, none, first, A->ctx->dev_err, 0,
                           gate));
         nk += 1;
@@ -1795,7 +1808,7 @@ hhp_status run_direct_mix(Solver *s, bool merged) {
                 HHP_CUDA(launch_k(k_s<float, true>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->S32, s->R32,
                                   s->V32, s->R0_32, nu4, parts_of(pl), s->part_s32));
                 HHP_TRY(launch_spmv32(A, st, EP_DOT3, s->S32, s->T32, s->S32, stop, s->R0_32));
-                HHP_CUDA(launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->X, s->D32, s->R32,
+                HHP_CUDA(launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, st, s->sc32, s->X, s->D32, s->R32,
                                   s->P32, s->S32, s->T32, s->V32, nu4, parts_of(pl), s->part_s32, s->nblk, s->hist,
                                   s->hist_cap, none, none, k == 0 ? 1 : 0, A->ctx->dev_err, 0));
             } else {
@@ -1806,7 +1819,7 @@ hhp_status run_direct_mix(Solver *s, bool merged) {
                                   s->S32, s->T32, s->R0_32, nu4, parts_of(pl), s->part_s32, s->nblk, s->part_xr32,
                                   static_cast<const float *>(s->S32)));
                 nk += 1;
-                HHP_CUDA(launch_k(k_p_ru, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->X, s->D32, s->P32, s->V32,
+                HHP_CUDA(launch_k(k_p_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, st, s->sc32, s->X, s->D32, s->P32, s->V32,
                                   s->R32, nu4, s->part_xr32, s->part_s32, s->nblk, s->hist, s->hist_cap, none, none,
                                   k == 0 ? 1 : 0, A->ctx->dev_err, 0));
             }
