@@ -92,6 +92,7 @@ constexpr int kLongGroup = 32;
 struct PlanDev {
     int rpl = 0, H = 0, n_slices = 0, n_long = 0, n_chunks = 0, ctas = 0, warps_per_cta = 0, unroll = 4;
     bool has_perm = false, sorted = false, d16 = false;  // d16: 16-bit column offsets (scol16)
+    bool deep = false;                // the longest slice is the critical path (see do_slice)
     bool uni = false;                 // uniform diagonals: no index stream, see uniform_diagonals
     int K = 0;                        // number of diagonals (slice width) when uni
     int doff[kMaxDiag] = {};          // their offsets col - row, ascending

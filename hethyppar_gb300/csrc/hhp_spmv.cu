@@ -43,6 +43,11 @@ namespace hhp {
 namespace {
 
 constexpr int kChunkUnroll = 4;
+// Length-sorted matrices whose longest slice is the critical path (PlanDev::deep): steps in flight at
+// once in its slices, and the resident CTAs that leaves. 8 steps on 3 CTAs against 4 on 5, FP64
+// power law, back to back: 40k rows 55 -> 33 us, 300k 72 -> 43, 1M 83 -> 54 (16 steps on 2 CTAs: 30, 41,
+// 61), 3.5M 138 -> 156.
+constexpr int kDeep = 8, kDeepCtas = 3;
 
 // A lane's words of one slice step: the values (V) and column indices (I: int32 columns; I16:
 // 16-bit offsets col - row) of its R rows, each read with one load (32 lanes make one contiguous
@@ -185,7 +190,7 @@ __device__ __forceinline__ void row_epilogue(const SellArgs<VT> &a, int r, VT ac
     }
 }
 
-template <typename VT, int R, int U, int EP, bool D16, bool UNI>
+template <typename VT, int R, int U, int EP, bool D16, bool UNI, bool DEEP>
 __device__ __forceinline__ void do_slice(const SellArgs<VT> &a, int s, long long base, int wmax, int lane,
                                          double &d0, double &d1, double &d2) {
     using VV = typename Vec<VT, R>::V;
@@ -282,17 +287,42 @@ __device__ __forceinline__ void do_slice(const SellArgs<VT> &a, int s, long long
     // Software pipeline over full groups of U steps: the values and indices of group g+1
     // are requested before the gathers and multiply-adds of group g, so the HBM latency of the
     // streams overlaps the L1/L2 latency of the gathers (warps issue in order: a load placed
-    // after a stalled FMA would wait for it). The last wmax % U steps run one at a time
-    // after the loop: a multiply-add predicated off still occupies GB300's FP64 pipe for a full
-    // warp slot, so no group is ever padded with dead steps.
+    // after a stalled FMA would wait for it). The last wmax % U steps follow the loop: a multiply-add
+    // predicated off still occupies GB300's FP64 pipe for a full warp slot, so no group is ever padded
+    // with dead steps.
+    int j = 0;
+    if constexpr (DEEP) {
+        // A slice of long rows is a chain: one gather latency per group of steps. With kDeep steps
+        // in a group the chain has half as many links; values are requested with the gathers.
+        constexpr int Q = kDeep;
+        if (wmax >= Q) {
+            CW cd[Q];
+#pragma unroll
+            for (int u = 0; u < Q; ++u) cd[u] = ld_stream<VT>(cp + static_cast<size_t>(u) * 32);
+            for (; j + Q <= wmax; j += Q) {
+                VV vd[Q];
+                VT xd[Q];
+#pragma unroll
+                for (int u = 0; u < Q; ++u) {
+                    vd[u] = ld_stream<VT>(vp + static_cast<size_t>(j + u) * 32);
+                    xd[u] = j + u < len[0] ? __ldg(a.x + colof(cd[u], 0)) : VT(0);
+                }
+#pragma unroll
+                for (int u = 0; u < Q; ++u)
+                    if (j + Q + u < wmax) cd[u] = ld_stream<VT>(cp + static_cast<size_t>(j + Q + u) * 32);
+#pragma unroll
+                for (int u = 0; u < Q; ++u)
+                    if (j + u < len[0]) acc[0] = vfma(comp<VV, VT>(vd[u], 0), xd[u], acc[0]);
+            }
+        }
+    }
     VV v[U];
     CW c[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-        v[u] = u < wmax ? ld_stream<VT>(vp + static_cast<size_t>(u) * 32) : VV();
-        c[u] = u < wmax ? ld_stream<VT>(cp + static_cast<size_t>(u) * 32) : CW();
+        v[u] = j + u < wmax ? ld_stream<VT>(vp + static_cast<size_t>(j + u) * 32) : VV();
+        c[u] = j + u < wmax ? ld_stream<VT>(cp + static_cast<size_t>(j + u) * 32) : CW();
     }
-    int j = 0;
     for (; j + U <= wmax; j += U) {
         VV vn[U];
         CW cn[U];
@@ -317,6 +347,28 @@ __device__ __forceinline__ void do_slice(const SellArgs<VT> &a, int s, long long
             v[u] = vn[u];
             c[u] = cn[u];
         }
+    }
+    // The last wmax % U steps. One row per lane (length-sorted power-law rows, whose lengths are all
+    // sizes): as one group of their own size, on the words that the last prefetch loaded, gathers
+    // together (3.5M rows: 146.5 -> 142.9 us). Two or four rows: one at a time; as a group they
+    // measured no faster (450k x 17: 24.8 vs 25.0 us) and the FP32 kernels spill.
+    if constexpr (R == 1) {
+        auto last = [&](auto n) {
+            constexpr int N = decltype(n)::value;
+            VT xt[N];
+#pragma unroll
+            for (int u = 0; u < N; ++u) xt[u] = j + u < len[0] ? __ldg(a.x + colof(c[u], 0)) : VT(0);
+#pragma unroll
+            for (int u = 0; u < N; ++u)
+                if (j + u < len[0]) acc[0] = vfma(comp<VV, VT>(v[u], 0), xt[u], acc[0]);
+        };
+        const int left = wmax - j;  // uniform across the warp
+        if constexpr (U > 2) {
+            if (left == 3) last(std::integral_constant<int, 3>());
+            if (left == 2) last(std::integral_constant<int, 2>());
+        }
+        if (left == 1) last(std::integral_constant<int, 1>());
+        j = wmax;
     }
     // tail steps, one at a time (their words were requested by the last prefetch)
 #pragma unroll 1
@@ -482,8 +534,8 @@ struct MinCtasFor {
     static constexpr int value = UNI && sizeof(VT) == 4 && R * U >= 8 ? 4 : MinCtas<R, U>::value;
 };
 
-template <typename VT, int R, int U, int EP, bool D16, bool UNI = false>
-__global__ void __launch_bounds__(256, MinCtasFor<VT, R, U, UNI>::value) k_spmv(const SellArgs<VT> a) {
+template <typename VT, int R, int U, int EP, bool D16, bool UNI = false, bool DEEP = false>
+__global__ void __launch_bounds__(256, DEEP ? kDeepCtas : MinCtasFor<VT, R, U, UNI>::value) k_spmv(const SellArgs<VT> a) {
     // After a recorded device error, with the gate closed, or once the solver's status is
     // terminal, the launch returns at once (uniform across the grid). The three words were
     // written by earlier launches: read together (one memory latency, not three), through L2.
@@ -504,7 +556,7 @@ __global__ void __launch_bounds__(256, MinCtasFor<VT, R, U, UNI>::value) k_spmv(
         if (u < a.n_slices) {
             const long long base = static_cast<long long>(static_cast<unsigned>(rec.z)) |
                                    (static_cast<long long>(rec.w) << 32);
-            do_slice<VT, R, U, EP, D16, UNI>(a, u, base, rec.y, lane, d0, d1, d2);
+            do_slice<VT, R, U, EP, D16, UNI, DEEP>(a, u, base, rec.y, lane, d0, d1, d2);
         } else {
             do_chunk<VT, EP>(a, u - a.n_slices, lane);
         }
@@ -626,19 +678,19 @@ cudaError_t launch_uni(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaS
     }
 }
 
-template <typename VT, int R, int U, bool D16, bool UNI = false>
+template <typename VT, int R, int U, bool D16, bool UNI = false, bool DEEP = false>
 cudaError_t launch_rud(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
     const dim3 grid(p.ctas), block(p.warps_per_cta * 32);
     switch (ep) {
-        case EP_DOT1: return launch_k(k_spmv<VT, R, U, EP_DOT1, D16, UNI>, grid, block, 0, s, a);
-        case EP_DOT2: return launch_k(k_spmv<VT, R, U, EP_DOT2, D16, UNI>, grid, block, 0, s, a);
-        case EP_DOT3: return launch_k(k_spmv<VT, R, U, EP_DOT3, D16, UNI>, grid, block, 0, s, a);
-        case EP_RESID: return launch_k(k_spmv<VT, R, U, EP_RESID, D16, UNI>, grid, block, 0, s, a);
+        case EP_DOT1: return launch_k(k_spmv<VT, R, U, EP_DOT1, D16, UNI, DEEP>, grid, block, 0, s, a);
+        case EP_DOT2: return launch_k(k_spmv<VT, R, U, EP_DOT2, D16, UNI, DEEP>, grid, block, 0, s, a);
+        case EP_DOT3: return launch_k(k_spmv<VT, R, U, EP_DOT3, D16, UNI, DEEP>, grid, block, 0, s, a);
+        case EP_RESID: return launch_k(k_spmv<VT, R, U, EP_RESID, D16, UNI, DEEP>, grid, block, 0, s, a);
         default:
             // y = A x needs no epilogue arithmetic: a separate instantiation keeps the FP64 pipe
             // free of predicated-off scale and accumulate instructions
-            if (!a.scale && !a.accum) return launch_k(k_spmv<VT, R, U, EP_Y, D16, UNI>, grid, block, 0, s, a);
-            return launch_k(k_spmv<VT, R, U, EP_AXPBY, D16, UNI>, grid, block, 0, s, a);
+            if (!a.scale && !a.accum) return launch_k(k_spmv<VT, R, U, EP_Y, D16, UNI, DEEP>, grid, block, 0, s, a);
+            return launch_k(k_spmv<VT, R, U, EP_AXPBY, D16, UNI, DEEP>, grid, block, 0, s, a);
     }
 }
 
@@ -663,6 +715,9 @@ cudaError_t launch_ep(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaSt
             return p.K == 5 ? launch_uni<VT, 4, 5, 4>(ep, p, a, s) : launch_uni<VT, 4, 7, 4>(ep, p, a, s);
     }
     if constexpr (std::is_same<VT, double>::value) {
+        if (p.deep)
+            return p.d16 ? launch_rud<VT, 1, 4, true, false, true>(ep, p, a, s)
+                         : launch_rud<VT, 1, 4, false, false, true>(ep, p, a, s);
         if (p.rpl == 1) return u2 ? launch_ru<VT, 1, 2>(ep, p, a, s) : launch_ru<VT, 1, 4>(ep, p, a, s);
         return u2 ? launch_ru<VT, 2, 2>(ep, p, a, s) : launch_ru<VT, 2, 4>(ep, p, a, s);
     } else {
@@ -823,6 +878,19 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
         }
     }
     if (uni && !std::is_same<VT, double>::value && R * U >= 8 && t.ctas_per_sm <= 0) cps = 4;
+    // One warp walks the longest slice, at ~0.2 us a step in groups of 4; the whole launch takes ~4 ps
+    // per nonzero (the L2's sector rate). Below 64000 nonzeros per step of the longest slice (16M at
+    // 256 steps) the walk is the longer of the two, and the launch takes the kernel with kDeep
+    // steps in flight on fewer CTAs (measured both ways at 8.6M: 83 -> 54 us, at 30M: 138 -> 156 us).
+    bool deep = false;
+    if (R == 1 && h.sorted) {
+        long long wmax = 0;
+        for (int s2 = 0; s2 < h.n_slices; ++s2)
+            wmax = std::max(wmax, (h.slice_ptr[static_cast<size_t>(s2) + 1] - h.slice_ptr[static_cast<size_t>(s2)]) / h.H);
+        deep = wmax >= kDeep && static_cast<long long>(A->nnz) < 64000 * wmax;
+        if (t.spmv_unroll != 0) deep = false;
+        if (deep && t.ctas_per_sm <= 0) cps = kDeepCtas;
+    }
     p.release();
     p.uni = uni;
     p.K = K;
@@ -836,6 +904,7 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
     for (int k = 0; k < kMaxDiag; ++k) p.doff[k] = doff[k];
     p.rpl = R;
     p.unroll = U;
+    p.deep = deep;
     p.H = h.H;
     p.n_slices = h.n_slices;
     p.n_long = static_cast<int>(h.long_rows.size());
