@@ -87,6 +87,12 @@ struct Solver {
     double *PH = nullptr, *SH = nullptr;
     cudaGraphExec_t g64i = nullptr, g64im = nullptr;
     long long g64i_gen = 0, g64im_gen = 0;
+    // one-kernel loop of small systems (k_small); grid 0: not for this system
+    double2 *RV = nullptr;
+    double *small_rec = nullptr;
+    unsigned *small_arrived = nullptr;
+    int small_grid = -1, small_rows = 0, small_k = 0, small_threads = 0;
+    bool small_cluster = false;  // grid -1: not decided yet
     int g64_kernels_pro = 0, g64_kernels_epi = 0, gmix_kernels_pro = 0, gmix_kernels_epi = 0, unroll = 4;
 };
 
@@ -781,6 +787,8 @@ __global__ void __launch_bounds__(512) k_xrp(DevScal *sc, T *X, T *R, T *P, cons
         unit(u, xx, pp, ss, tt, vx, pxx, sxx);
     }
 }
+
+#include "hhp_small.cuh"
 
 // Final true residual (SpMV EP_RESID into Y already done): ||b - A x||^2, ||b||^2.
 __global__ void k_finish(DevScal *sc, SpmvParts sp) {
@@ -1577,6 +1585,126 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
     return end_loop_body(s, st);
 }
 
+cudaLaunchConfig_t small_config(int blocks, int threads, size_t smem, bool cluster, cudaStream_t st,
+                                cudaLaunchAttribute *attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(blocks));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    if (cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = cfg.gridDim.x;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+
+using SmallKernel = void (*)(const SmallArgs);
+SmallKernel small_kernel(bool merged, bool cluster) {
+    return merged ? (cluster ? k_small<true, true> : k_small<true, false>)
+                  : (cluster ? k_small<false, true> : k_small<false, false>);
+}
+
+// Decides once per matrix whether its FP64 loop runs as k_small, and lays out what that needs: fewer
+// than 65,536 rows (from there on the loop is the graph's 4 or 5 launches an iteration, whose number
+// callers rely on; k_small would be the faster one up to its limit of 512 rows per block, 77,824: 270^2
+// stencil 15.5 against 20.5 us), rows in natural order (no long or length-sorted ones: a row is one
+// thread's) of at most kSmallMaxK entries, and the blocks' entries in shared memory.
+constexpr int kSmallRows = 65535;
+
+hhp_status ensure_small(Solver *s) {
+    if (s->small_grid >= 0) return HHP_OK;
+    hhp_mat *A = s->A;
+    HHP_TRY(ensure_plan(A, false));
+    const PlanDev &p = A->plan64;
+    s->small_grid = 0;
+    if (A->n > kSmallRows || p.has_perm) return HHP_OK;
+    int k = 1;
+    for (int i = 0; i < A->m; ++i)
+        k = std::max(k, A->rowptr_host[static_cast<size_t>(i) + 1] - A->rowptr_host[static_cast<size_t>(i)]);
+    bool cluster = A->n <= kSmallClusterRows;
+    int blocks = 1;
+    if (cluster) {  // a power of two, 32 rows per block at least
+        while (blocks < kSmallCluster && blocks * 32 < A->n) blocks *= 2;
+    } else {
+        blocks = std::min(A->ctx->num_sms, kSmallMaxGrid);
+    }
+    const int rows = (A->n + blocks - 1) / blocks;
+    int threads = 32;  // a power of two (the reduction tree), a row each
+    while (threads < rows) threads *= 2;
+    const size_t smem = static_cast<size_t>(k) * static_cast<size_t>(rows) * 12;
+    if (k > kSmallMaxK || threads > kSmallThreads || smem + sizeof(SmallShared) + 1024 > A->ctx->smem_optin) return HHP_OK;
+    for (const SmallKernel kern : {small_kernel(true, cluster), small_kernel(false, cluster)}) {
+        HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        int fit = 0;  // every block has to be resident
+        if (cluster) {
+            HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            cudaLaunchAttribute attr[1];
+            const cudaLaunchConfig_t cfg = small_config(blocks, threads, smem, true, A->ctx->stream, attr);
+            if (cudaOccupancyMaxActiveClusters(&fit, kern, &cfg) != cudaSuccess) fit = 0;
+        } else if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kern, threads, smem) != cudaSuccess) {
+            fit = 0;
+        }
+        if (fit < 1) {
+            cudaGetLastError();
+            return HHP_OK;  // the graph loop, then
+        }
+    }
+    hhp_status st = HHP_OK;
+    s->RV = dalloc<double2>(static_cast<size_t>(s->n_pad), st, A->ctx->stream);
+    s->small_rec = dalloc<double>(2 * kSmallQ * kSmallMaxGrid, st, A->ctx->stream);
+    s->small_arrived = dalloc<unsigned>(1, st, A->ctx->stream);
+    HHP_TRY(st);
+    s->small_rows = rows;
+    s->small_k = k;
+    s->small_cluster = cluster;
+    s->small_threads = threads;
+    s->small_grid = blocks;
+    return HHP_OK;
+}
+
+hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
+    hhp_mat *A = s->A;
+    const PlanDev &p = A->plan64;
+    SmallArgs a;
+    a.sc = s->sc;
+    a.slice_ptr = p.slice_ptr;
+    a.pos_len = p.pos_len;
+    a.sval = static_cast<const double *>(p.sval);
+    a.scol = p.scol;
+    a.scol16 = p.scol16;
+    a.uni = p.uni ? 1 : 0;
+    a.nd = p.K;
+    a.H = p.H;
+    a.K = s->small_k;
+    a.n = A->n;
+    a.rows = s->small_rows;
+    for (int k = 0; k < kMaxDiag; ++k) a.doff[k] = p.doff[k];
+    a.X = s->X;
+    a.P = s->P;
+    a.S = s->S;
+    a.R = s->R;
+    a.RV = s->RV;
+    a.rec = s->small_rec;
+    a.arrived = s->small_arrived;
+    a.hist = s->hist;
+    a.hist_cap = s->hist_cap;
+    a.dev_err = A->ctx->dev_err;
+    cudaLaunchAttribute attr[1];
+    const cudaLaunchConfig_t cfg =
+        small_config(s->small_grid, s->small_threads, static_cast<size_t>(s->small_k) * static_cast<size_t>(s->small_rows) * 12,
+                     s->small_cluster, st, attr);
+    if (!s->small_cluster) HHP_CUDA(cudaMemsetAsync(s->small_arrived, 0, sizeof(unsigned), st));
+    HHP_CUDA(cudaLaunchKernelEx(&cfg, small_kernel(merged, s->small_cluster), a));
+    return HHP_OK;
+}
+
 // Zeroes the x0 flag and runs k_x0check on `st` (captured into the solve graphs).
 hhp_status launch_x0check(Solver *s, cudaStream_t st) {
     HHP_CUDA(cudaMemsetAsync(s->x0_nz, 0, sizeof(int), st));
@@ -1607,8 +1735,14 @@ hhp_status run_direct64(Solver *s, bool merged, bool ilu) {
         A->ctx->kernel_launches += 1;
         return HHP_OK;
     };
-    if (merged) HHP_TRY(kp(0));  // stop tests on the initial residual
-    for (;;) {
+    const bool small = !ilu && s->small_grid > 0;
+    if (small) {
+        HHP_TRY(launch_small(s, st, merged));
+        A->ctx->kernel_launches += 1;
+    } else if (merged) {
+        HHP_TRY(kp(0));  // stop tests on the initial residual
+    }
+    while (!small) {
         for (int k = 0; k < s->unroll; ++k) {
             if (merged) {
                 const double *pv = s->P, *sv = s->S;
@@ -1685,8 +1819,10 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
         if (rc != HHP_OK) break;
         HHP_CUDA(launch_k(k_init<double>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc, s->R, s->B, s->R0, s->P, s->V,
                           nu, parts_of(A->plan64), s->x0_nz, s->part_b, s->nblk, s->part_xr, s->part_s));
-        rc = capture_loop<double>(s, st, s->sc, s->X, s->R, s->R0, s->P, s->V, s->S, s->T, s->part_xr, s->part_s,
-                                  false, merged, ilu);
+        const bool small = !ilu && s->small_grid > 0;
+        rc = small ? launch_small(s, st, merged)
+                   : capture_loop<double>(s, st, s->sc, s->X, s->R, s->R0, s->P, s->V, s->S, s->T, s->part_xr,
+                                          s->part_s, false, merged, ilu);
         if (rc != HHP_OK) break;
         rc = launch_spmv64(A, st, EP_RESID, s->X, s->Y, s->B, 1.0, 0.0);
         if (rc != HHP_OK) break;
@@ -1707,7 +1843,7 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
     s->g64_kernels_epi = 2;
     // launch_spmv64 / launch_ilu_apply counted their captured launches; graph launches are counted
     // when executed.
-    A->ctx->kernel_launches -= 2 + (ilu ? 6 : 2) * s->unroll;
+    A->ctx->kernel_launches -= 2 + (!ilu && s->small_grid > 0 ? 0 : (ilu ? 6 : 2) * s->unroll);
     if (ilu) (merged ? s->g64im_gen : s->g64i_gen) = ilu_generation(A);
     return HHP_OK;
 }
@@ -1951,6 +2087,7 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
         // resolved AUTO to CLASSIC before it gets here
         // (ILU(0) adds its two applications, 4 kernels, to either schedule)
         const bool merged = o->loop != HHP_LOOP_CLASSIC && !h.fixed;
+        if (!ilu) HHP_TRY(ensure_small(s));
         cudaGraphExec_t &ge = ilu ? (merged ? s->g64im : s->g64i) : merged ? s->g64m : s->g64;
         if (use_graph && !ge) HHP_TRY(build_g64(s, merged, ilu));
         const long long per_iter = (merged ? 4 : 5) + (ilu ? 4 : 0);
@@ -2105,6 +2242,9 @@ void solver_release(Solver *s) {
     double *d[] = {s->X, s->B, s->R, s->R0, s->P, s->V, s->S, s->T, s->Y, s->part_xr, s->part_s, s->part_xr32,
                    s->part_s32, s->part_b, s->hist, s->PH, s->SH};
     cudaFree(s->x0_nz);
+    cudaFree(s->RV);
+    cudaFree(s->small_rec);
+    cudaFree(s->small_arrived);
     for (double *p : d) cudaFree(p);
     float *f[] = {s->D32, s->R32, s->R0_32, s->P32, s->V32, s->S32, s->T32};
     for (float *p : f) cudaFree(p);
