@@ -1611,12 +1611,13 @@ SmallKernel small_kernel(bool merged, bool cluster) {
                   : (cluster ? k_small<false, true> : k_small<false, false>);
 }
 
-// Decides once per matrix whether its FP64 loop runs as k_small, and lays out what that needs: fewer
-// than 65,536 rows (from there on the loop is the graph's 4 or 5 launches an iteration, whose number
-// callers rely on; k_small would be the faster one up to its limit of 512 rows per block, 77,824: 270^2
-// stencil 15.5 against 20.5 us), rows in natural order (no long or length-sorted ones: a row is one
-// thread's) of at most kSmallMaxK entries, and the blocks' entries in shared memory.
-constexpr int kSmallRows = 65535;
+// Decides once per matrix whether its FP64 loop runs as k_small, and lays out what that needs: at most
+// kSmallRows rows, in natural order (no long or length-sorted ones: a row is one thread's), of at most
+// kSmallMaxK entries, and the blocks' entries in shared memory. The gain over the graph loop falls with
+// the size (5-point stencils: 1.9x at 8,100 rows, 1.7x at 16,384, 1.34x at 62,500), as the FP64 work per
+// SM grows; the line lies where it is about 1.5x, so that the loop of a system of tens of thousands of
+// rows and more keeps its summation order and its 4 or 5 launches an iteration.
+constexpr int kSmallRows = 40000;
 
 hhp_status ensure_small(Solver *s) {
     if (s->small_grid >= 0) return HHP_OK;

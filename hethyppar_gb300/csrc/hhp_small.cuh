@@ -1,10 +1,10 @@
 // hhp_small.cuh -- the FP64 BiCGStab loop of a small system as one cooperative kernel.
 //
 // 5-point stencils, us an iteration against the graph loop: 32^2 7.9 / 19.4, 64^2 9.1 / 19.7, 128^2
-// 11.7 / 20.1, 250^2 15.4 / 20.7 (classic 64^2 10.1 / 25.0); 17 entries per row: 20,000 rows 17.9 /
-// 30.0, 60,000 rows 23.2 / 31.6.
+// 11.7 / 20.1 (classic 64^2 10.1 / 25.0); 17 entries per row: 4,000 rows 14.0 / 27.5, 20,000 rows
+// 17.9 / 30.0.
 //
-// Below some tens of thousands of rows an iteration of the graph loop is 4 (classic: 5) launches of
+// On a system of few rows an iteration of the graph loop is 4 (classic: 5) launches of
 // ~5 us each, nearly all of it launch gaps and chains of latencies: the work list, the partial
 // records, operands that left the registers a kernel ago. Here the whole system lives on the SMs: a
 // row per thread, its matrix entries in shared memory, its elements of x, r, r0, p, v, s and t in
