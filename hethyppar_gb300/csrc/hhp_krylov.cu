@@ -1612,8 +1612,7 @@ SmallKernel small_kernel(bool merged, bool cluster) {
 }
 
 // Decides once per matrix whether its FP64 loop runs as k_small, and lays out what that needs: at most
-// kSmallRows rows, in natural order (no long or length-sorted ones: a row is one thread's), of at most
-// kSmallMaxK entries, and the blocks' entries in shared memory. The gain over the graph loop falls with
+// kSmallRows rows, none of them cut into chunks (a row is one thread's), of at most kSmallMaxK entries, and the blocks' entries in shared memory. The gain over the graph loop falls with
 // the size (5-point stencils: 1.9x at 8,100 rows, 1.7x at 16,384, 1.34x at 62,500), as the FP64 work per
 // SM grows; the line lies where it is about 1.5x, so that the loop of a system of tens of thousands of
 // rows and more keeps its summation order and its 4 or 5 launches an iteration.
@@ -1625,7 +1624,7 @@ hhp_status ensure_small(Solver *s) {
     HHP_TRY(ensure_plan(A, false));
     const PlanDev &p = A->plan64;
     s->small_grid = 0;
-    if (A->n > kSmallRows || p.has_perm) return HHP_OK;
+    if (A->n > kSmallRows || p.n_long > 0) return HHP_OK;
     int k = 1;
     for (int i = 0; i < A->m; ++i)
         k = std::max(k, A->rowptr_host[static_cast<size_t>(i) + 1] - A->rowptr_host[static_cast<size_t>(i)]);
@@ -1676,6 +1675,7 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
     SmallArgs a;
     a.sc = s->sc;
     a.slice_ptr = p.slice_ptr;
+    a.pos_row = p.has_perm ? p.pos_row : nullptr;
     a.pos_len = p.pos_len;
     a.sval = static_cast<const double *>(p.sval);
     a.scol = p.scol;

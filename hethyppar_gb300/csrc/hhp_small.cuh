@@ -18,15 +18,15 @@
 //
 // Up to kSmallClusterRows rows the blocks are one thread-block cluster: an exchange is partial sums
 // pushed into every block's shared memory and the hardware's cluster barrier (556 cycles at 16
-// blocks). Above that the FP64 work of 16 SMs outweighs the cheaper exchange: the grid is launched cooperatively (all blocks resident) and an exchange
-// is records in L2 and an arrival count that every block polls (1.2 us; polling all blocks' records
-// instead took 3.3 us at 152 blocks). Every such wait is bounded: one that runs out sets the
+// blocks). Above that the FP64 work of 16 SMs outweighs the cheaper exchange: the grid is launched
+// cooperatively (all blocks resident) and an exchange is records in L2 and an arrival count that every
+// block polls (1.2 us; polling all blocks' records instead took 3.3 us at 152 blocks). Every such wait is bounded: one that runs out sets the
 // context's error word and the block leaves, as the others then do. All blocks add the same numbers in
 // the same order, so they compute the same scalars bit for bit and take the same branches.
 #pragma once
 
 constexpr int kSmallThreads = 512;
-constexpr int kSmallMaxK = 32;            // entries per row, at most
+constexpr int kSmallMaxK = 64;            // entries per row, at most
 constexpr int kSmallPubS = 9;             // above: t = A s gathers published s (an exchange costs what
                                           // some ten FP64 instructions of every warp do)
 constexpr int kSmallQ = 5;                // quantities of the widest exchange
@@ -40,6 +40,7 @@ constexpr int kSmallPolls = 1 << 20;      // reads of the count before giving up
 struct SmallArgs {
     DevScal *sc;
     const long long *slice_ptr;
+    const int *pos_row;       // the row at each position of the slices (null: the position)
     const int *pos_len;       // row lengths, or masks of diagonals (uni)
     const double *sval;
     const int *scol;
@@ -163,8 +164,9 @@ template <bool MERGED, bool CLUSTER>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constant__ SmallArgs a) {
     extern __shared__ double s_mat[];  // val[K][rows], then col[K][rows]
     __shared__ SmallShared sh;
-    const int t = threadIdx.x, row = blockIdx.x * a.rows + t;
-    const bool own = t < a.rows && row < a.n, lead = blockIdx.x == 0 && t == 0;
+    const int t = threadIdx.x, pos = blockIdx.x * a.rows + t;
+    const bool own = t < a.rows && pos < a.n, lead = blockIdx.x == 0 && t == 0;
+    const int row = own && a.pos_row ? a.pos_row[pos] : pos;
     double *sv = s_mat + t;
     int *sc_ = reinterpret_cast<int *>(s_mat + a.K * a.rows) + t;
     const int ld = a.rows;
@@ -177,9 +179,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
     int len = 0;
     double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, tv = 0.0;
     if (own) {
-        const long long base = a.uni ? static_cast<long long>(row / a.H) * a.nd * a.H + row % a.H
-                                     : a.slice_ptr[row / a.H] + row % a.H;
-        const int pl = a.pos_len[row];
+        const long long base = a.uni ? static_cast<long long>(pos / a.H) * a.nd * a.H + pos % a.H
+                                     : a.slice_ptr[pos / a.H] + pos % a.H;
+        const int pl = a.pos_len[pos];
         if (a.uni) {
             for (int k = 0; k < a.nd; ++k)
                 if (pl >> k & 1) {
@@ -202,16 +204,31 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
         a.RV[row].x = r;
     }
     const double r0 = r;
-    // sum over the row's entries, in order, of val * get(col): eight gathers in flight
+    // sum over the row's entries, in order, of val * get(col): eight gathers in flight, as many steps as
+    // the warp's longest row has (a multiply-add that no lane needs still takes the FP64 pipe's slot)
+    const int kmax = __reduce_max_sync(0xffffffffu, len);
     auto row_sum = [&](auto get) {
         double acc = 0.0;
-        for (int k = 0; k < a.K; k += 8) {
-            double g[8];
+        auto steps = [&](auto n, int k) {
+            constexpr int N = decltype(n)::value;
+            double g[N];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) g[u] = k + u < len ? get(sc_[(k + u) * ld]) : 0.0;
+            for (int u = 0; u < N; ++u) g[u] = k + u < len ? get(sc_[(k + u) * ld]) : 0.0;
 #pragma unroll
-            for (int u = 0; u < 8; ++u)
+            for (int u = 0; u < N; ++u)
                 if (k + u < len) acc = fma(sv[(k + u) * ld], g[u], acc);
+        };
+        int k = 0;
+        for (; k + 8 <= kmax; k += 8) steps(std::integral_constant<int, 8>(), k);
+        switch (kmax - k) {
+            case 1: steps(std::integral_constant<int, 1>(), k); break;
+            case 2: steps(std::integral_constant<int, 2>(), k); break;
+            case 3: steps(std::integral_constant<int, 3>(), k); break;
+            case 4: steps(std::integral_constant<int, 4>(), k); break;
+            case 5: steps(std::integral_constant<int, 5>(), k); break;
+            case 6: steps(std::integral_constant<int, 6>(), k); break;
+            case 7: steps(std::integral_constant<int, 7>(), k); break;
+            default: break;
         }
         return acc;
     };

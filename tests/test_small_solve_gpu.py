@@ -7,7 +7,7 @@ import math
 import numpy as np
 import pytest
 
-from hethyppar_gb300 import Matrix, bicgstab, synth
+from hethyppar_gb300 import Matrix, bicgstab, bicgstab_backward, synth
 from oracle import oracle as orc
 
 pytestmark = pytest.mark.gpu
@@ -53,6 +53,37 @@ def test_sizes(ctx, m, width, loop):
     assert np.array_equal(x, x2) and r.iters == r2.iters
     xz, rz = bicgstab(ctx, A, b, rtol=1e-11, loop=loop)
     assert rz.status == 0 and _rel(rp, col, val, b, xz) <= 1.0000001e-11
+    A.close()
+
+
+@pytest.mark.parametrize("m", [50, 3000, 20_000])
+@pytest.mark.parametrize("loop", ["merged", "classic"])
+def test_length_sorted_rows(ctx, m, loop):
+    """Row lengths from 1 to 31: the layout sorts them, a thread's row is not its position."""
+    rng = np.random.default_rng(m)
+    lens = np.minimum(rng.choice([1, 2, 3, 9, 17, 31], size=m), m)
+    cols = []
+    for i, n in enumerate(lens):
+        c = rng.choice(m, size=n - 1, replace=False)
+        cols.append(np.concatenate([np.sort(c[c != i]), [i]]))
+    rp = np.concatenate([[0], np.cumsum([c.size for c in cols])]).astype(np.int32)
+    col = np.concatenate(cols).astype(np.int32)
+    val = rng.uniform(-1.0, 0.0, col.size)
+    rows = np.repeat(np.arange(m), np.diff(rp))
+    off = np.bincount(rows[col != rows], weights=np.abs(val[col != rows]), minlength=m)
+    val[col == rows] = 1.3 * off + 0.5
+    b = rng.standard_normal(m)
+    A = Matrix.from_csr(ctx, rp, col, val)
+    # (no bar on the count here: on these systems it moves by 10% with the summation order)
+    x, r = bicgstab(ctx, A, b, rtol=1e-11, loop=loop, maxit=300)
+    assert r.status == 0 and _rel(rp, col, val, b, x) <= 1.0000001e-11
+    # the transpose, whose rows are sorted differently, as the adjoint solves it
+    g = rng.standard_normal(m)
+    dldb, dlda, ra = bicgstab_backward(ctx, A, x, g, rtol=1e-11, maxit=300, loop=loop)
+    tr, tc, tv = orc.csr_to_csc(rp, col, val, m)
+    assert ra.status == 0 and _rel(tr, tc, tv, g, dldb) <= 1.0000001e-11
+    rows = np.repeat(np.arange(m), np.diff(rp))
+    assert np.array_equal(dlda, -(dldb[rows] * x[col]))
     A.close()
 
 
