@@ -65,6 +65,7 @@ struct Solver {
     // threads per block of the kernels without dot products (K_P, K_XRP and their mixed forms), per
     // vector unit type; see update_threads
     int nthr_u64 = 512, nthr_u32 = 512;
+    bool narrow32 = false;  // see kNarrow
     // FP64 vectors (n_pad each)
     double *X = nullptr, *B = nullptr, *R = nullptr, *R0 = nullptr, *P = nullptr, *V = nullptr, *S = nullptr,
            *T = nullptr, *Y = nullptr;
@@ -265,6 +266,13 @@ __device__ __forceinline__ int step_p(int status, int iter, int it0, int maxit, 
 constexpr int kPre = 4;
 constexpr int kPreX = 3;
 constexpr int kPreXPC = 2;  // K_XRP with right preconditioning: seven operand streams
+// The mixed form's merged K_S and K_XRP_RU on vectors of at most kNarrowUnits units: blocks of kNarrow
+// threads with kPreNarrow units in flight each, the same bytes in flight from half the warps, whose
+// barriers and reductions cost half (us an inner iteration, 512 threads / this: 256^2 5-point 20.1 /
+// 19.1, 1024^2 37.5 / 35.7, 100^3 7-point 45.3 / 43.2, 125^3 62.4 / 60.7; 140^3, where the
+// vectors come from HBM, 79.7 / 84.1). FP64 kernels measured no faster so (1024^2 72.9 / 74.5), and their
+// dot products keep their order.
+constexpr int kNarrow = 256, kPreNarrow = 6, kNarrowUnits = 1 << 19;
 
 // Scalar work (divisions, tests) is done once per block by thread 0 and broadcast through shared
 // memory: on GB300 an FP64 division is a sequence of FP64 instructions on the slowest pipe, so
@@ -389,8 +397,8 @@ __global__ void __launch_bounds__(512) k_p(DevScal *sc, T *P, const T *V, const 
 
 // K_S: alpha = rho / (r0.v), s = r - alpha v, partial s.s. Merged loop (M): also r0.s, in
 // records of 4 (s.s, r0.s, 0, 0) for K_XRP.
-template <typename T, bool M = false>
-__global__ void __launch_bounds__(512) k_s(DevScal *sc, T *S, const T *R, const T *V, const T *R0, int nu,
+template <typename T, bool M = false, int NT = 512>
+__global__ void __launch_bounds__(NT) k_s(DevScal *sc, T *S, const T *R, const T *V, const T *R0, int nu,
                                            SpmvParts sp, double *part_s) {
     const bool dead = dead_step(sc);  // tested after the operand and record loads are in flight
     // scalars written by earlier launches, read with the operand loads (off the critical path)
@@ -400,7 +408,8 @@ __global__ void __launch_bounds__(512) k_s(DevScal *sc, T *S, const T *R, const 
     __shared__ double bc[1];
     __shared__ int go;
     constexpr int E = Unit<T>::E;
-    constexpr int KP = M ? kPreX : kPre;  // three vectors' operands in the merged form
+    // three vectors' operands in the merged form; in half the threads twice as many units each
+    constexpr int KP = NT == kNarrow ? kPreNarrow : M ? kPreX : kPre;
     const int stride = gridDim.x * blockDim.x, u0 = blockIdx.x * blockDim.x + threadIdx.x;
     T r[KP][E], vv[KP][E], q[M ? KP : 1][E];
 #pragma unroll
@@ -993,7 +1002,8 @@ __global__ void __launch_bounds__(512) k_p_ru(DevScal *sc, double *X, float *D32
 // r = s - omega t, beta, p = r + beta (p - omega v). With one: x += d + alpha p + omega s, d = 0,
 // and the IF node runs the FP64 residual, the residual replacement and K_P (r and p are left to
 // it). Divergence or a vanished t.t / rho ends the pass as a breakdown with d not folded.
-__global__ void __launch_bounds__(512) k_xrp_ru(DevScal *sc, double *X, float *D32, float *R, float *P, const float *S,
+template <int NT>
+__global__ void __launch_bounds__(NT) k_xrp_ru(DevScal *sc, double *X, float *D32, float *R, float *P, const float *S,
                                                 const float *Tv, const float *V, int nu4, SpmvParts sp,
                                                 const double *part_s, int nparts, double *hist, int hist_cap,
                                                 cudaGraphConditionalHandle wcond, cudaGraphConditionalHandle icond,
@@ -1009,10 +1019,11 @@ __global__ void __launch_bounds__(512) k_xrp_ru(DevScal *sc, double *X, float *D
     __shared__ double red[kRedScratch];
     __shared__ float bc[3];
     __shared__ int go;  // 0: nothing, 1: d, r, p updates, 2: fold d + alpha p + omega s into x
+    constexpr int KX = NT == kNarrow ? kPreNarrow : kPreX;
     const int stride = gridDim.x * blockDim.x, u0 = blockIdx.x * blockDim.x + threadIdx.x;
-    float d[kPreX][4], p[kPreX][4], s[kPreX][4], t[kPreX][4], vv[kPreX][4];
+    float d[KX][4], p[KX][4], s[KX][4], t[KX][4], vv[KX][4];
 #pragma unroll
-    for (int k = 0; k < kPreX; ++k) {
+    for (int k = 0; k < KX; ++k) {
         const int u = u0 + k * stride;
         if (u < nu4) {
             ldu(d[k], D32, u);
@@ -1128,15 +1139,15 @@ __global__ void __launch_bounds__(512) k_xrp_ru(DevScal *sc, double *X, float *D
         stu(P, u, pp);
     };
 #pragma unroll
-    for (int k = 0; k < kPreX; ++k) {
+    for (int k = 0; k < KX; ++k) {
         const int u = u0 + k * stride;
         if (u < nu4) unit(u, d[k], p[k], s[k], t[k], vv[k]);
     }
-    // whole batches of kPreX units, then the last few one at a time (see K_P)
-    int ub = u0 + kPreX * stride;
-    for (; ub + (kPreX - 1) * stride < nu4; ub += kPreX * stride) {
+    // whole batches of KX units, then the last few one at a time (see K_P)
+    int ub = u0 + KX * stride;
+    for (; ub + (KX - 1) * stride < nu4; ub += KX * stride) {
 #pragma unroll
-        for (int k = 0; k < kPreX; ++k) {
+        for (int k = 0; k < KX; ++k) {
             ldu(d[k], D32, ub + k * stride);
             ldu(p[k], P, ub + k * stride);
             ldu(s[k], S, ub + k * stride);
@@ -1144,7 +1155,7 @@ __global__ void __launch_bounds__(512) k_xrp_ru(DevScal *sc, double *X, float *D
             ldu(vv[k], V, ub + k * stride);
         }
 #pragma unroll
-        for (int k = 0; k < kPreX; ++k) unit(ub + k * stride, d[k], p[k], s[k], t[k], vv[k]);
+        for (int k = 0; k < KX; ++k) unit(ub + k * stride, d[k], p[k], s[k], t[k], vv[k]);
     }
     for (int u = ub; u < nu4; u += stride) {
         float dd[4], pp[4], ss[4], tt[4], vx[4];
@@ -1258,6 +1269,7 @@ hhp_status ensure_solver(hhp_mat *A, Solver **out, int maxit) {
         s->unroll = std::max(1, std::min(tuning().unroll_iters, 16));
         s->nthr_u64 = update_threads(s->nblk, s->n_pad / 2);
         s->nthr_u32 = update_threads(s->nblk, s->n_pad / 4);
+        s->narrow32 = s->n_pad / 4 <= kNarrowUnits;
         hhp_status st = HHP_OK;
         const size_t np = static_cast<size_t>(s->n_pad);
         s->X = dalloc<double>(np, st, A->ctx->stream);
@@ -1481,14 +1493,16 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
             }
             st = launch_spmv32(A, s->s2, EP_DOT1, P, V, R0, stop);
             if (st != HHP_OK) break;
-            if (launch_k(k_s<float, true>, dim3(s->nblk), dim3(s->nthr), 0, s->s2, sc, S, R, V, R0, nu,
+            if (launch_k(s->narrow32 ? k_s<float, true, kNarrow> : k_s<float, true>, dim3(s->nblk),
+                         dim3(s->narrow32 ? kNarrow : s->nthr), 0, s->s2, sc, S, R, V, R0, nu,
                          parts_of(pl), part_s) != cudaSuccess) {
                 st = HHP_ERR_CUDA;
                 break;
             }
             st = launch_spmv32(A, s->s2, EP_DOT3, S, Tv, S, stop, R0);
             if (st != HHP_OK) break;
-            if (launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, s->s2, s->sc32, s->X, s->D32, s->R32, s->P32,
+            if (launch_k(s->narrow32 ? k_xrp_ru<kNarrow> : k_xrp_ru<512>, dim3(s->nblk),
+                         dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, s->s2, s->sc32, s->X, s->D32, s->R32, s->P32,
                          s->S32, s->T32, s->V32, nu4, parts_of(pl), part_s, s->nblk, s->hist, s->hist_cap, cond,
                          icond_body, k == 0 ? 1 : 0, A->ctx->dev_err, 1) != cudaSuccess) {
                 st = HHP_ERR_CUDA;
@@ -1942,10 +1956,12 @@ hhp_status run_direct_mix(Solver *s, bool merged) {
         for (int k = 0; k < s->unroll; ++k) {
             HHP_TRY(launch_spmv32(A, st, EP_DOT1, s->P32, s->V32, s->R0_32, stop));
             if (merged) {
-                HHP_CUDA(launch_k(k_s<float, true>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->S32, s->R32,
+                HHP_CUDA(launch_k(s->narrow32 ? k_s<float, true, kNarrow> : k_s<float, true>, dim3(s->nblk),
+                         dim3(s->narrow32 ? kNarrow : s->nthr), 0, st, s->sc32, s->S32, s->R32,
                                   s->V32, s->R0_32, nu4, parts_of(pl), s->part_s32));
                 HHP_TRY(launch_spmv32(A, st, EP_DOT3, s->S32, s->T32, s->S32, stop, s->R0_32));
-                HHP_CUDA(launch_k(k_xrp_ru, dim3(s->nblk), dim3(s->nthr_u32), 0, st, s->sc32, s->X, s->D32, s->R32,
+                HHP_CUDA(launch_k(s->narrow32 ? k_xrp_ru<kNarrow> : k_xrp_ru<512>, dim3(s->nblk),
+                         dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, st, s->sc32, s->X, s->D32, s->R32,
                                   s->P32, s->S32, s->T32, s->V32, nu4, parts_of(pl), s->part_s32, s->nblk, s->hist,
                                   s->hist_cap, none, none, k == 0 ? 1 : 0, A->ctx->dev_err, 0));
             } else {
