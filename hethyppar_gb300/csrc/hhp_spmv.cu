@@ -43,6 +43,7 @@ namespace hhp {
 namespace {
 
 constexpr int kChunkUnroll = 4;
+constexpr long long kStreamKeep = 96LL << 20;  // of the 129 MB L2
 // Length-sorted matrices whose longest slice is the critical path (PlanDev::deep): steps in flight at
 // once in its slices, and the resident CTAs that leaves. 8 steps on 3 CTAs against 4 on 5, FP64
 // power law, back to back: 40k rows 55 -> 33 us, 300k 72 -> 43, 1M 83 -> 54 (16 steps on 2 CTAs: 30, 41,
@@ -580,6 +581,24 @@ __device__ __forceinline__ void load_run(VT (&o)[N], const VT *x, int i, int off
     for (int t = 0; t < N; ++t) o[t] = __ldg(x + i + t);
 }
 
+// The value stream's words in k_spmv_uni. ONCE: with an evict-first hint, in the FP32 loop's products on
+// matrices whose stream fills the L2 (kStreamKeep): the solve's vectors then stay there between its
+// kernels (160^3, 115 MB: DRAM reads of the mixed form's K_S 33 -> 11 MB, of K_XRP_RU 74 -> 44 MB, an
+// inner iteration 108.6 -> 105.2 us). A plain product has nothing to keep and a shorter stream is
+// better kept itself (28.2 -> 30 us; 1024^2 FP64 back to back 14.4 -> 16.0); the FP64 kernels have no
+// registers left for the policy.
+template <bool ONCE, typename T>
+__device__ __forceinline__ T ld_value(const T *p, uint64_t policy) {
+    if constexpr (ONCE) {
+        static_assert(std::is_same<T, float2>::value, "the FP32 kernel's words");
+        float2 v;
+        asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(policy));
+        return v;
+    } else {
+        return __ldg(p);
+    }
+}
+
 // Uniform diagonals, K = 5 or 7 of them (2D and 3D stencils). The general kernel reads such a slice in
 // dependent rounds (work record, masks, a group of values and gathers, the last K mod U steps one by
 // one); here nothing waits for anything but the multiply-adds:
@@ -594,7 +613,7 @@ __device__ __forceinline__ void load_run(VT (&o)[N], const VT *x, int i, int off
 // Lanes own the same rows and units as in the general kernel, so the dot products' partial sums are
 // the same too, bit for bit. 160^3 7-point: FP32 32.8 -> 28.4 us (the mixed solve 119.8 -> 108.7 us
 // an iteration), FP64 60.2 -> 58.5 us; 256^2 5-point FP64 6.2 -> 4.2 us (23.0 -> 21.7 us a solve iteration).
-template <typename VT, int R, int K, int EP, int CTAS>
+template <typename VT, int R, int K, int EP, int CTAS, bool ONCE = false>
 __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ SellArgs<VT> a) {
     constexpr int H = 32 * R, N = R / 2;  // N rows per lane and pass
     using VN = typename Vec<VT, N>::V;
@@ -605,6 +624,8 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
     const int gw = blockIdx.x * nw + warp, W = gridDim.x * nw;
     const int err = __ldcg(a.err), gate = a.gate ? __ldcg(a.gate) : 1, stop = a.stop ? __ldcg(a.stop) : 0;
     const bool skip = err != DEV_OK || gate == 0 || stop != 0;
+    uint64_t policy = 0;
+    if constexpr (ONCE) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int u = gw; u < a.n_slices; u += W) {
         const int q0 = u * H + lane * R;
@@ -620,7 +641,7 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
             VN v[K];
             VT xv[K][N];
 #pragma unroll
-            for (int k = 0; k < K; ++k) v[k] = __ldg(reinterpret_cast<const VN *>(vp + k * H + N * h));
+            for (int k = 0; k < K; ++k) v[k] = ld_value<ONCE>(reinterpret_cast<const VN *>(vp + k * H + N * h), policy);
             if (safe) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) load_run<VT, N>(xv[k], a.x, q0 + N * h + a.doff[k], a.doff[k], a.x_vec);
@@ -667,6 +688,16 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
 template <typename VT, int R, int K, int CTAS>
 cudaError_t launch_uni(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
     const dim3 grid(p.ctas), block(p.warps_per_cta * 32);
+    if constexpr (std::is_same<VT, float>::value) {
+        if (p.total * static_cast<long long>(sizeof(VT)) > kStreamKeep) {
+            switch (ep) {
+                case EP_DOT1: return launch_k(k_spmv_uni<VT, R, K, EP_DOT1, CTAS, true>, grid, block, 0, s, a);
+                case EP_DOT2: return launch_k(k_spmv_uni<VT, R, K, EP_DOT2, CTAS, true>, grid, block, 0, s, a);
+                case EP_DOT3: return launch_k(k_spmv_uni<VT, R, K, EP_DOT3, CTAS, true>, grid, block, 0, s, a);
+                default: break;
+            }
+        }
+    }
     switch (ep) {
         case EP_DOT1: return launch_k(k_spmv_uni<VT, R, K, EP_DOT1, CTAS>, grid, block, 0, s, a);
         case EP_DOT2: return launch_k(k_spmv_uni<VT, R, K, EP_DOT2, CTAS>, grid, block, 0, s, a);
