@@ -47,7 +47,7 @@ constexpr long long kStreamKeep = 96LL << 20;  // of the 129 MB L2
 // Length-sorted matrices whose longest slice is the critical path (PlanDev::deep): steps in flight at
 // once in its slices, and the resident CTAs that leaves. 8 steps on 3 CTAs against 4 on 5, FP64
 // power law, back to back: 40k rows 55 -> 33 us, 300k 72 -> 43, 1M 83 -> 54 (16 steps on 2 CTAs: 30, 41,
-// 61), 3.5M 138 -> 156.
+// 61), 3.5M 138 -> 156. FP32 (2 rows per lane): 40k 26 -> 20.5, 300k 45 -> 42, 1M 78 -> 66.
 constexpr int kDeep = 8, kDeepCtas = 3;
 
 // A lane's words of one slice step: the values (V) and column indices (I: int32 columns; I16:
@@ -302,18 +302,21 @@ __device__ __forceinline__ void do_slice(const SellArgs<VT> &a, int s, long long
             for (int u = 0; u < Q; ++u) cd[u] = ld_stream<VT>(cp + static_cast<size_t>(u) * 32);
             for (; j + Q <= wmax; j += Q) {
                 VV vd[Q];
-                VT xd[Q];
+                VT xd[Q][R];
 #pragma unroll
                 for (int u = 0; u < Q; ++u) {
                     vd[u] = ld_stream<VT>(vp + static_cast<size_t>(j + u) * 32);
-                    xd[u] = j + u < len[0] ? __ldg(a.x + colof(cd[u], 0)) : VT(0);
+#pragma unroll
+                    for (int t = 0; t < R; ++t) xd[u][t] = j + u < len[t] ? __ldg(a.x + colof(cd[u], t)) : VT(0);
                 }
 #pragma unroll
                 for (int u = 0; u < Q; ++u)
                     if (j + Q + u < wmax) cd[u] = ld_stream<VT>(cp + static_cast<size_t>(j + Q + u) * 32);
 #pragma unroll
                 for (int u = 0; u < Q; ++u)
-                    if (j + u < len[0]) acc[0] = vfma(comp<VV, VT>(vd[u], 0), xd[u], acc[0]);
+#pragma unroll
+                    for (int t = 0; t < R; ++t)
+                        if (j + u < len[t]) acc[t] = vfma(comp<VV, VT>(vd[u], t), xd[u][t], acc[t]);
             }
         }
     }
@@ -752,6 +755,9 @@ cudaError_t launch_ep(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaSt
         if (p.rpl == 1) return u2 ? launch_ru<VT, 1, 2>(ep, p, a, s) : launch_ru<VT, 1, 4>(ep, p, a, s);
         return u2 ? launch_ru<VT, 2, 2>(ep, p, a, s) : launch_ru<VT, 2, 4>(ep, p, a, s);
     } else {
+        if (p.deep)
+            return p.d16 ? launch_rud<VT, 2, 4, true, false, true>(ep, p, a, s)
+                         : launch_rud<VT, 2, 4, false, false, true>(ep, p, a, s);
         if (p.rpl == 2) return u2 ? launch_ru<VT, 2, 2>(ep, p, a, s) : launch_ru<VT, 2, 4>(ep, p, a, s);
         return u2 ? launch_ru<VT, 4, 2>(ep, p, a, s) : launch_ru<VT, 4, 4>(ep, p, a, s);
     }
@@ -877,6 +883,15 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
         cps = t.ctas_per_sm > 0 ? t.ctas_per_sm : 3;
         build_plan(A->m, A->rowptr_host.data(), R, std::max(t.long_thr, 1), std::max(t.cap, 32),
                    std::max(t.window, 1), h);
+        // length-sorted rows: 2 per lane on 4 CTAs, shorter chains in the slices of long rows and more
+        // warps for the gathers (power law, back to back: 40k rows 35 -> 25 us, 300k 62 -> 45, 3.5M 153
+        // -> 137)
+        if (h.sorted && R == 4 && t.rpl32 != 2) {
+            R = 2;
+            if (t.ctas_per_sm <= 0) cps = 4;
+            build_plan(A->m, A->rowptr_host.data(), R, std::max(t.long_thr, 1), std::max(t.cap, 32),
+                       std::max(t.window, 1), h);
+        }
     }
     // Uniform diagonals (stencils): every entry on one of at most kMaxDiag diagonals, rows in
     // natural order, no long rows. The slices then store values only, K steps each (step k =
@@ -914,7 +929,7 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
     // 256 steps) the walk is the longer of the two, and the launch takes the kernel with kDeep
     // steps in flight on fewer CTAs (measured both ways at 8.6M: 83 -> 54 us, at 30M: 138 -> 156 us).
     bool deep = false;
-    if (R == 1 && h.sorted) {
+    if (R == (std::is_same<VT, double>::value ? 1 : 2) && h.sorted) {
         long long wmax = 0;
         for (int s2 = 0; s2 < h.n_slices; ++s2)
             wmax = std::max(wmax, (h.slice_ptr[static_cast<size_t>(s2) + 1] - h.slice_ptr[static_cast<size_t>(s2)]) / h.H);

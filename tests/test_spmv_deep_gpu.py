@@ -1,9 +1,11 @@
-"""FP64 SpMV of length-sorted matrices: rows at the edges of the groups of steps (4 and 8), of the
+"""SpMV (FP64 and FP32) of length-sorted matrices: rows at the edges of the groups of steps (4 and 8), of the
 slice limit (256 entries) and of the chunks beyond it, on short matrices (the deep kernel) and on a
 long one (the ordinary one), with all epilogues through a solve."""
 import numpy as np
 import pytest
+import torch
 
+from gpu_util import dev
 from hethyppar_gb300 import Matrix, bicgstab
 from oracle import oracle as orc
 
@@ -35,6 +37,14 @@ def test_rows_at_the_edges(ctx, m, pool, far):
     assert np.array_equal(y[short], ref[short])
     bound = 2.0 * np.diff(rp) * 2.3e-16 * orc.spmv(rp, col, np.abs(val), np.abs(x))
     assert np.all(np.abs(y - ref) <= bound)
+    # FP32: at most one rounding per entry of a partial sum of magnitude sum |a x|, one for the store
+    x32, v32 = x.astype(np.float32), val.astype(np.float32)
+    exact = orc.spmv(rp, col, v32.astype(np.float64), x32.astype(np.float64))
+    bound = (np.diff(rp) + 1) * 2.0 ** -24 * 1.01 * orc.spmv(rp, col, np.abs(v32).astype(np.float64),
+                                                             np.abs(x32).astype(np.float64))
+    y32 = torch.empty(m, dtype=torch.float32, device="cuda")
+    A.spmv_f32_dev(dev(x32, torch.float32), y32)
+    assert np.all(np.abs(y32.cpu().numpy() - exact) <= bound)
     A.close()
 
 
@@ -53,6 +63,10 @@ def test_solve_on_edge_rows(ctx, loop):
     b = np.random.default_rng(2).standard_normal(m)
     A = Matrix.from_csr(ctx, rp2, c2, v2)
     x, r = bicgstab(ctx, A, b, rtol=1e-12, loop=loop)
+    assert r.status == 0
+    res = b - orc.spmv(rp2, c2, v2, x)
+    assert np.sqrt(orc.dot(res, res) / orc.dot(b, b)) <= 1.0000001e-12
+    x, r = bicgstab(ctx, A, b, rtol=1e-12, loop=loop, precision="mixed")
     assert r.status == 0
     res = b - orc.spmv(rp2, c2, v2, x)
     assert np.sqrt(orc.dot(res, res) / orc.dot(b, b)) <= 1.0000001e-12
