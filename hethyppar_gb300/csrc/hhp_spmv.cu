@@ -43,7 +43,7 @@ namespace hhp {
 namespace {
 
 constexpr int kChunkUnroll = 4;
-constexpr long long kStreamKeep = 96LL << 20;  // of the 129 MB L2
+constexpr long long kStreamKeep = 100LL << 20;  // of the 129 MB L2
 // Length-sorted matrices whose longest slice is the critical path (PlanDev::deep): steps in flight at
 // once in its slices, and the resident CTAs that leaves. 8 steps on 3 CTAs against 4 on 5, FP64
 // power law, back to back: 40k rows 55 -> 33 us, 300k 72 -> 43, 1M 83 -> 54 (16 steps on 2 CTAs: 30, 41,
@@ -584,22 +584,17 @@ __device__ __forceinline__ void load_run(VT (&o)[N], const VT *x, int i, int off
     for (int t = 0; t < N; ++t) o[t] = __ldg(x + i + t);
 }
 
-// The value stream's words in k_spmv_uni. ONCE: with an evict-first hint, in the FP32 loop's products on
-// matrices whose stream fills the L2 (kStreamKeep): the solve's vectors then stay there between its
-// kernels (160^3, 115 MB: DRAM reads of the mixed form's K_S 33 -> 11 MB, of K_XRP_RU 74 -> 44 MB, an
-// inner iteration 108.6 -> 105.2 us). A plain product has nothing to keep and a shorter stream is
-// better kept itself (28.2 -> 30 us; 1024^2 FP64 back to back 14.4 -> 16.0); the FP64 kernels have no
-// registers left for the policy.
+// The value stream's words in k_spmv_uni. ONCE (streaming loads, first out of the caches): in the solve
+// loop's products where the stream and the loop's vectors together do not fit the L2 (kStreamKeep); the
+// vectors then stay there between its kernels. 160^3 mixed: DRAM reads of K_S 33 -> 11 MB, of
+// K_XRP_RU 74 -> 44 MB, an inner iteration 109.2 -> 103.7 us; 140^3 79.0 -> 72.8, 125^3 58.9 -> 57.0; FP64
+// 1024^2 73.8 -> 72.9. Where all fits it costs 3 % (100^3 mixed, 60 MB: 38.6 -> 39.9), and a plain product
+// has no vectors to keep. (An evict-first policy operand did the same in FP32, less well: 105.2; the
+// FP64 kernels have no registers for it.)
 template <bool ONCE, typename T>
-__device__ __forceinline__ T ld_value(const T *p, uint64_t policy) {
-    if constexpr (ONCE) {
-        static_assert(std::is_same<T, float2>::value, "the FP32 kernel's words");
-        float2 v;
-        asm("ld.global.nc.L2::cache_hint.v2.f32 {%0, %1}, [%2], %3;" : "=f"(v.x), "=f"(v.y) : "l"(p), "l"(policy));
-        return v;
-    } else {
-        return __ldg(p);
-    }
+__device__ __forceinline__ T ld_value(const T *p) {
+    if constexpr (ONCE) return __ldcs(p);
+    else return __ldg(p);
 }
 
 // Uniform diagonals, K = 5 or 7 of them (2D and 3D stencils). The general kernel reads such a slice in
@@ -627,8 +622,6 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
     const int gw = blockIdx.x * nw + warp, W = gridDim.x * nw;
     const int err = __ldcg(a.err), gate = a.gate ? __ldcg(a.gate) : 1, stop = a.stop ? __ldcg(a.stop) : 0;
     const bool skip = err != DEV_OK || gate == 0 || stop != 0;
-    uint64_t policy = 0;
-    if constexpr (ONCE) asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int u = gw; u < a.n_slices; u += W) {
         const int q0 = u * H + lane * R;
@@ -644,7 +637,7 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
             VN v[K];
             VT xv[K][N];
 #pragma unroll
-            for (int k = 0; k < K; ++k) v[k] = ld_value<ONCE>(reinterpret_cast<const VN *>(vp + k * H + N * h), policy);
+            for (int k = 0; k < K; ++k) v[k] = ld_value<ONCE>(reinterpret_cast<const VN *>(vp + k * H + N * h));
             if (safe) {
 #pragma unroll
                 for (int k = 0; k < K; ++k) load_run<VT, N>(xv[k], a.x, q0 + N * h + a.doff[k], a.doff[k], a.x_vec);
@@ -691,14 +684,12 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
 template <typename VT, int R, int K, int CTAS>
 cudaError_t launch_uni(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
     const dim3 grid(p.ctas), block(p.warps_per_cta * 32);
-    if constexpr (std::is_same<VT, float>::value) {
-        if (p.total * static_cast<long long>(sizeof(VT)) > kStreamKeep) {
-            switch (ep) {
-                case EP_DOT1: return launch_k(k_spmv_uni<VT, R, K, EP_DOT1, CTAS, true>, grid, block, 0, s, a);
-                case EP_DOT2: return launch_k(k_spmv_uni<VT, R, K, EP_DOT2, CTAS, true>, grid, block, 0, s, a);
-                case EP_DOT3: return launch_k(k_spmv_uni<VT, R, K, EP_DOT3, CTAS, true>, grid, block, 0, s, a);
-                default: break;
-            }
+    if ((p.total + 8LL * a.m) * static_cast<long long>(sizeof(VT)) > kStreamKeep) {
+        switch (ep) {
+            case EP_DOT1: return launch_k(k_spmv_uni<VT, R, K, EP_DOT1, CTAS, true>, grid, block, 0, s, a);
+            case EP_DOT2: return launch_k(k_spmv_uni<VT, R, K, EP_DOT2, CTAS, true>, grid, block, 0, s, a);
+            case EP_DOT3: return launch_k(k_spmv_uni<VT, R, K, EP_DOT3, CTAS, true>, grid, block, 0, s, a);
+            default: break;
         }
     }
     switch (ep) {
@@ -909,7 +900,12 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
         hc.resize(static_cast<size_t>(A->nnz));
         HHP_CUDA(cudaStreamSynchronize(ctx->stream));
         HHP_CUDA(cudaMemcpy(hc.data(), A->col, sizeof(int) * n_pre, cudaMemcpyDeviceToHost));
-        if (uniform_diagonals(m_pre, rp.data(), hc.data(), kMaxDiag, 0.10, doff, K, mask)) {
+        // FP32: the prefix may hold any number of absent entries, as the first rows of a grid lie on its
+        // boundary (11,000 rows of a 100^3 grid are its first plane and a tenth, 13 % padding; the mixed
+        // solve 44.2 -> 38.6 us an iteration). FP64 leaves such grids to 16-bit offsets, with which
+        // their solves are faster (100^3: 77.1 against 79.1 us an iteration).
+        const double pad = std::is_same<VT, double>::value ? 0.10 : 1e9;
+        if (uniform_diagonals(m_pre, rp.data(), hc.data(), kMaxDiag, pad, doff, K, mask)) {
             HHP_CUDA(cudaMemcpy(hc.data() + n_pre, A->col + n_pre, sizeof(int) * (hc.size() - n_pre),
                                 cudaMemcpyDeviceToHost));
             uni = uniform_diagonals(A->m, rp.data(), hc.data(), kMaxDiag, 0.10, doff, K, mask);
