@@ -78,6 +78,7 @@ struct Solver {
     double *part_xr32 = nullptr, *part_s32 = nullptr;  // nblk*2 each (FP32 inner loop)
     DevScal *sc = nullptr, *sc32 = nullptr;            // device
     DevScal *h_sc = nullptr, *h_sc32 = nullptr;        // pinned host mirrors
+    int *h_err = nullptr;                              // the context's error word after a pass (pinned)
     double *hist = nullptr;
     int hist_cap = 0;
     cudaStream_t s2 = nullptr, s3 = nullptr;  // capture streams: loop body, IF body
@@ -1291,6 +1292,7 @@ hhp_status ensure_solver(hhp_mat *A, Solver **out, int maxit) {
         s->sc32 = dalloc<DevScal>(1, st, A->ctx->stream);
         if (st == HHP_OK && cudaMallocHost(&s->h_sc, sizeof(DevScal)) != cudaSuccess) st = HHP_ERR_OOM;
         if (st == HHP_OK && cudaMallocHost(&s->h_sc32, sizeof(DevScal)) != cudaSuccess) st = HHP_ERR_OOM;
+        if (st == HHP_OK && cudaMallocHost(&s->h_err, sizeof(int)) != cudaSuccess) st = HHP_ERR_OOM;
         if (st == HHP_OK && (cudaStreamCreateWithFlags(&s->s2, cudaStreamNonBlocking) != cudaSuccess ||
                              cudaStreamCreateWithFlags(&s->s3, cudaStreamNonBlocking) != cudaSuccess ||
                              cudaEventCreateWithFlags(&s->ev_in, cudaEventDisableTiming) != cudaSuccess))
@@ -1704,7 +1706,7 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
     a.X = s->X;
     a.P = s->P;
     a.S = s->S;
-    a.R = s->R;
+    a.B = s->B;
     a.RV = s->RV;
     a.rec = s->small_rec;
     a.arrived = s->small_arrived;
@@ -1737,6 +1739,11 @@ hhp_status run_direct64(Solver *s, bool merged, bool ilu) {
     const int nu = s->n_pad / 2;
     const int *stop = &s->sc->status;
     HHP_CUDA(cudaMemcpyAsync(s->sc, s->h_sc, kCtlBytes, cudaMemcpyHostToDevice, st));
+    if (!ilu && s->small_grid > 0) {
+        HHP_TRY(launch_small(s, st, merged));
+        A->ctx->kernel_launches += 1;
+        return HHP_OK;
+    }
     HHP_TRY(launch_x0check(s, st));
     HHP_TRY(launch_spmv64(A, st, EP_RESID, s->X, s->R, s->B, 1.0, 0.0, s->x0_nz));
     HHP_CUDA(launch_k(k_init<double>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc, s->R, s->B, s->R0, s->P, s->V, nu,
@@ -1750,14 +1757,8 @@ hhp_status run_direct64(Solver *s, bool merged, bool ilu) {
         A->ctx->kernel_launches += 1;
         return HHP_OK;
     };
-    const bool small = !ilu && s->small_grid > 0;
-    if (small) {
-        HHP_TRY(launch_small(s, st, merged));
-        A->ctx->kernel_launches += 1;
-    } else if (merged) {
-        HHP_TRY(kp(0));  // stop tests on the initial residual
-    }
-    while (!small) {
+    if (merged) HHP_TRY(kp(0));  // stop tests on the initial residual
+    for (;;) {
         for (int k = 0; k < s->unroll; ++k) {
             if (merged) {
                 const double *pv = s->P, *sv = s->S;
@@ -1821,11 +1822,16 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
     cudaStream_t st = A->ctx->stream;
     HHP_TRY(ensure_plan(A, false));
     const int nu = s->n_pad / 2;
+    const bool small = !ilu && s->small_grid > 0;
     HHP_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     hhp_status rc = HHP_OK;
     do {
         if (cudaMemcpyAsync(s->sc, s->h_sc, kCtlBytes, cudaMemcpyHostToDevice, st) != cudaSuccess) {
             rc = HHP_ERR_CUDA;
+            break;
+        }
+        if (small) {  // one kernel for the whole pass
+            rc = launch_small(s, st, merged);
             break;
         }
         rc = launch_x0check(s, st);
@@ -1834,10 +1840,8 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
         if (rc != HHP_OK) break;
         HHP_CUDA(launch_k(k_init<double>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc, s->R, s->B, s->R0, s->P, s->V,
                           nu, parts_of(A->plan64), s->x0_nz, s->part_b, s->nblk, s->part_xr, s->part_s));
-        const bool small = !ilu && s->small_grid > 0;
-        rc = small ? launch_small(s, st, merged)
-                   : capture_loop<double>(s, st, s->sc, s->X, s->R, s->R0, s->P, s->V, s->S, s->T, s->part_xr,
-                                          s->part_s, false, merged, ilu);
+        rc = capture_loop<double>(s, st, s->sc, s->X, s->R, s->R0, s->P, s->V, s->S, s->T, s->part_xr, s->part_s,
+                                  false, merged, ilu);
         if (rc != HHP_OK) break;
         rc = launch_spmv64(A, st, EP_RESID, s->X, s->Y, s->B, 1.0, 0.0);
         if (rc != HHP_OK) break;
@@ -1858,7 +1862,7 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
     s->g64_kernels_epi = 2;
     // launch_spmv64 / launch_ilu_apply counted their captured launches; graph launches are counted
     // when executed.
-    A->ctx->kernel_launches -= 2 + (!ilu && s->small_grid > 0 ? 0 : (ilu ? 6 : 2) * s->unroll);
+    if (!small) A->ctx->kernel_launches -= 2 + (ilu ? 6 : 2) * s->unroll;
     if (ilu) (merged ? s->g64im_gen : s->g64i_gen) = ilu_generation(A);
     return HHP_OK;
 }
@@ -2071,7 +2075,8 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
         HHP_TRY(copy_in(s->X, x_io, A->n, st, host));
     }
     HHP_CUDA(cudaEventRecord(ctx->ev0, st));
-    int dev_err = 0;
+    int &dev_err = *s->h_err;  // pinned: a copy to pageable memory would be staged and waited for
+    dev_err = DEV_OK;
     // After each pass: end-of-solve event, the iterate out to the caller, the device scalars and
     // the error word back -- one synchronisation for all (a restart repeats them).
     auto readback = [&](DevScal *hs, const DevScal *ds) -> hhp_status {
@@ -2122,7 +2127,9 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
             HHP_TRY(readback(s->h_sc, s->sc));
             ++outer;
             if (use_graph)
-                ctx->kernel_launches += s->g64_kernels_pro + s->g64_kernels_epi + per_iter * s->unroll * h.bodies;
+                ctx->kernel_launches += !ilu && s->small_grid > 0
+                                            ? 1
+                                            : s->g64_kernels_pro + s->g64_kernels_epi + per_iter * s->unroll * h.bodies;
             dev_status = h.status;
             // Residual replacement: the recursive residual met the threshold but the true one
             // did not (rounding drift); restart from the current iterate, whose true residual
@@ -2269,6 +2276,7 @@ void solver_release(Solver *s) {
     cudaFree(s->sc32);
     cudaFreeHost(s->h_sc);
     cudaFreeHost(s->h_sc32);
+    cudaFreeHost(s->h_err);
     if (s->s2) cudaStreamDestroy(s->s2);
     if (s->s3) cudaStreamDestroy(s->s3);
     if (s->ev_in) cudaEventDestroy(s->ev_in);

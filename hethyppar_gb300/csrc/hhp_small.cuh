@@ -8,7 +8,8 @@
 // ~5 us each, nearly all of it launch gaps and chains of latencies: the work list, the partial
 // records, operands that left the registers a kernel ago. Here the whole system lives on the SMs: a
 // row per thread, its matrix entries in shared memory, its elements of x, r, r0, p, v, s and t in
-// registers; what other rows need (p, and r with v, or s) goes through L2. An iteration has three grid-wide
+// registers; what other rows need (p, and r with v, or s) goes through L2. The initial and the final
+// residual are formed here too, so a solve is this one launch. An iteration has three grid-wide
 // exchanges (classic: four):
 //   v = A p               -> sum of r0.v                      (and every v is visible)
 //   s = r - alpha v, t = A s -> sums of t.s, t.t, r0.t, s.s, r0.s
@@ -48,7 +49,7 @@ struct SmallArgs {
     int uni, nd, H, K, n, rows;  // rows: of a block
     int doff[kMaxDiag];
     double *X, *P, *S;
-    const double *R;
+    const double *B;
     double2 *RV;              // {r, v}
     double *rec;              // 2 sets of kSmallQ * grid partial sums, used in turn
     unsigned *arrived;        // blocks that have arrived, over all exchanges (zero at the launch)
@@ -171,13 +172,15 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
     int *sc_ = reinterpret_cast<int *>(s_mat + a.K * a.rows) + t;
     const int ld = a.rows;
     DevScal *sc = a.sc;
-    const double thr2 = sc->thr2_rec;
-    const int maxit = sc->maxit, it0 = sc->iter_start;
+    // control words, and on a restart the counts and threshold of the passes before (the lead thread
+    // writes them at the end, which no block reaches before all have taken part in the first exchange)
+    const int restart = sc->restart, maxit = sc->maxit, fixed = sc->fixed;
+    const double rtol2 = sc->rtol2, thr2_in = sc->thr2, rr0_in = sc->rr0;
+    const int it0 = restart ? sc->iter : 0;
     unsigned e = 0;
-    int iter = it0, status = sc->status;
-    double rr = sc->rr_last, rho = rr, alpha = 1.0, omega = 1.0;
+    int iter = it0, status = ST_RUNNING;
     int len = 0;
-    double x = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, tv = 0.0;
+    double x = 0.0, b = 0.0, r = 0.0, p = 0.0, v = 0.0, s = 0.0, tv = 0.0;
     if (own) {
         const long long base = a.uni ? static_cast<long long>(pos / a.H) * a.nd * a.H + pos % a.H
                                      : a.slice_ptr[pos / a.H] + pos % a.H;
@@ -198,12 +201,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
             len = pl;
         }
         x = a.X[row];
-        r = a.R[row];
-        p = r;
-        a.P[row] = p;
-        a.RV[row].x = r;
+        b = a.B[row];
     }
-    const double r0 = r;
     // sum over the row's entries, in order, of val * get(col): eight gathers in flight, as many steps as
     // the warp's longest row has (a multiply-add that no lane needs still takes the FP64 pipe's slot)
     const int kmax = __reduce_max_sync(0xffffffffu, len);
@@ -233,14 +232,34 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
         return acc;
     };
     const double none[1] = {0.0};
-    // stop tests on the initial residual (K_P's first run)
-    if (status == ST_RUNNING) {
-        if (thr2 >= 0.0 && rr <= thr2) status = ST_CONVERGED;
-        else if (iter >= maxit) status = ST_MAXIT;
-        else if (!finite_nonzero(rho) || !isfinite(rr)) status = ST_BREAKDOWN;
+    // r = b - A x, p = r; ||r||^2, ||b||^2 and whether x0 has a nonzero. x0 = 0 means r = b, also where
+    // A holds an infinity or a NaN (the loop finds it): formed again then.
+    r = b - row_sum([&](int c) { return __ldcg(a.X + c); });
+    auto publish = [&] {
+        p = r;
+        if (own) {
+            a.P[row] = p;
+            a.RV[row].x = r;
+        }
+    };
+    publish();
+    const double di[3] = {own ? r * r : 0.0, own ? b * b : 0.0, own && x != 0.0 ? 1.0 : 0.0};
+    bool good = exchange<3, CLUSTER>(a, sh, di, e);
+    double rr = sh.tot[0], alpha = 1.0, omega = 1.0;
+    const double bb = sh.tot[1], thr2 = restart ? thr2_in : fixed ? -1.0 : rtol2 * bb;
+    if (good && !isfinite(rr) && sh.tot[2] == 0.0) {
+        r = b;
+        rr = bb;
+        publish();
+        good = exchange<0, CLUSTER>(a, sh, none, e);
     }
-    bool good = true;
-    if (status == ST_RUNNING) good = exchange<0, CLUSTER>(a, sh, none, e);
+    const double r0 = r;
+    double rho = rr;
+    // stop tests on the initial residual (K_P's first run)
+    if (thr2 >= 0.0 && rr <= thr2) status = ST_CONVERGED;
+    else if (iter >= maxit) status = ST_MAXIT;
+    else if (!finite_nonzero(rho) || !isfinite(rr)) status = ST_BREAKDOWN;
+    __syncthreads();  // sh.tot has been read
     while (status == ST_RUNNING && good) {
         // v = A p, alpha
         v = row_sum([&](int c) { return __ldcg(a.P + c); });
@@ -390,9 +409,25 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
         good = exchange<0, CLUSTER>(a, sh, none, e);
     }
     if (own) a.X[row] = x;
+    // the true residual of the result
+    double true_rr = rr;
+    if (good) good = exchange<0, CLUSTER>(a, sh, none, e);
+    if (good) {
+        const double res = b - row_sum([&](int c) { return __ldcg(a.X + c); });
+        const double df[1] = {own ? res * res : 0.0};
+        good = exchange<1, CLUSTER>(a, sh, df, e);
+        true_rr = sh.tot[0];
+    }
     if (lead) {
         sc->status = good ? status : ST_DEVICE_ERROR;
+        sc->rr0 = restart ? rr0_in : bb;
+        sc->thr2 = sc->thr2_rec = thr2;
+        sc->bb = bb;
         sc->iter = iter;
+        sc->iter_start = it0;
+        sc->bodies = 0;
+        sc->arrivals = 0;
         sc->rr_last = rr;
+        sc->true_rr = true_rr;
     }
 }

@@ -136,3 +136,18 @@ def test_fixed_iterations(ctx):
     assert r.iters == 12 and r.status == 0
     assert np.max(np.abs(x - ref)) <= 1e-10 * np.max(np.abs(ref))
     A.close()
+
+
+@pytest.mark.parametrize("m", [500, 20_000, 40_001])
+@pytest.mark.parametrize("loop", ["merged", "classic"])
+def test_infinite_entry(ctx, m, loop):
+    """From x0 = 0 the residual is b whatever A holds, so the iterate stays 0; from another x0 it is not finite."""
+    rp, col, val = _dominant(m, 4, m)
+    val[rp[m // 2]] = np.inf
+    b = np.random.default_rng(m).standard_normal(m)
+    A = Matrix.from_csr(ctx, rp, col, val)
+    x, r = bicgstab(ctx, A, b, rtol=1e-10, loop=loop, raise_on_error=False)
+    assert r.status == 5 and r.iters == 0 and np.array_equal(x, np.zeros(m))
+    x, r = bicgstab(ctx, A, b, np.ones(m), rtol=1e-10, loop=loop, raise_on_error=False)
+    assert r.status == 5 and r.iters == 0 and np.array_equal(x, np.ones(m))
+    A.close()
