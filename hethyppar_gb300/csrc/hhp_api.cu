@@ -141,19 +141,19 @@ hhp_status csr_needed(const hhp_mat *A, const char *what) {
     return HHP_ERR_STATE;
 }
 
-hhp_status mat_refresh_derived(hhp_mat *A) {
+hhp_status mat_refresh_derived(hhp_mat *A, bool make32) {
     HHP_TRY(csr_needed(A, "the FP32 value copy"));
-    if (!A->val32) {
+    if (!A->val32 && make32) {
         HHP_CUDA(cudaMalloc(&A->val32, (static_cast<size_t>(A->nnz) + 4) * sizeof(float)));
         HHP_CUDA(cudaMemsetAsync(A->val32, 0, (static_cast<size_t>(A->nnz) + 4) * sizeof(float), A->ctx->stream));
     }
-    if (A->nnz > 0) {
+    if (A->val32 && A->nnz > 0) {
         const int grid = static_cast<int>(std::max(1LL, std::min((A->nnz + 255LL) / 256, 8LL * A->ctx->num_sms)));
         k_to_f32<<<grid, 256, 0, A->ctx->stream>>>(A->val, A->val32, A->nnz);
         HHP_CUDA(cudaGetLastError());
     }
     HHP_TRY(refresh_plan_values(A));
-    if (A->t) HHP_TRY(refresh_transpose_values(A));
+    if (A->t) HHP_TRY(refresh_transpose_values(A, make32));
     return HHP_OK;
 }
 
@@ -451,7 +451,8 @@ static hhp_status set_values(hhp_mat *A, const double *v, cudaMemcpyKind kind) {
     HHP_TRY(csr_needed(A, "hhp_mat_set_values"));
     if (A->nnz > 0)
         HHP_CUDA(cudaMemcpyAsync(A->val, v, sizeof(double) * static_cast<size_t>(A->nnz), kind, A->ctx->stream));
-    if (A->val32 || A->t || A->plan64.built() || A->plan32.built()) HHP_TRY(mat_refresh_derived(A));
+    // (what exists is brought up to date; the FP32 values are first made when something needs them)
+    if (A->val32 || A->t || A->plan64.built() || A->plan32.built()) HHP_TRY(mat_refresh_derived(A, false));
     HHP_CUDA(cudaStreamSynchronize(A->ctx->stream));
     release_jacobi(A);  // rebuilt from the new values on the next preconditioned solve
     release_ilu(A);

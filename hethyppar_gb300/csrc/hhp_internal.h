@@ -242,7 +242,7 @@ hhp_status backward_dev(hhp_mat *A, const double *x_dev, const double *g_dev, do
 
 // ---- transpose (hhp_transpose.cu) -----------------------------------------------------------------
 hhp_status ensure_transpose(hhp_mat *A);
-hhp_status refresh_transpose_values(hhp_mat *A);
+hhp_status refresh_transpose_values(hhp_mat *A, bool make32);
 hhp_status launch_dlda(hhp_mat *A, cudaStream_t s, const double *lambda, const double *x, double *dlda);
 
 // ---- files (hhp_io.cpp) ----------------------------------------------------------------------------
@@ -251,7 +251,7 @@ hhp_status read_mtx(const char *path, int &m, int &n, int &nnz, std::vector<int>
 
 // ---- matrix helpers (hhp_api.cpp) ------------------------------------------------------------------
 hhp_status mat_create_dev(hhp_ctx *ctx, int m, int n, int nnz, hhp_mat **out);  // allocates, zero padding
-hhp_status mat_refresh_derived(hhp_mat *A);                                      // after value changes
+hhp_status mat_refresh_derived(hhp_mat *A, bool make32 = true);  // after value changes; make32: FP32 values too
 inline int pad4(int n) { return (n + 3) & ~3; }
 
 // Kernel tuning knobs (environment overrides read once).

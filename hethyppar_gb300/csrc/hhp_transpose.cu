@@ -234,12 +234,12 @@ hhp_status ensure_transpose(hhp_mat *A) {
     return HHP_OK;
 }
 
-hhp_status refresh_transpose_values(hhp_mat *A) {
+hhp_status refresh_transpose_values(hhp_mat *A, bool make32) {
     if (!A->t) return HHP_OK;
     if (A->nnz > 0)
         k_t_vals<<<grid_for(A->ctx, A->nnz, 256), 256, 0, A->ctx->stream>>>(A->t_map, A->val, A->nnz, A->t->val);
     HHP_CUDA(cudaGetLastError());
-    return mat_refresh_derived(A->t);
+    return mat_refresh_derived(A->t, make32);
 }
 
 hhp_status launch_dlda(hhp_mat *A, cudaStream_t s, const double *lambda, const double *x, double *dlda) {
