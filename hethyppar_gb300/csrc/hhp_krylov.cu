@@ -883,14 +883,6 @@ __global__ void __launch_bounds__(512) k_mix_init(DevScal *sc, const double *Yd,
     }
 }
 
-// Growth of the FP32 recursive ||r||^2 over the last true ||b - A x||^2 taken as divergence
-// (a factor 1e5 in the norm: BiCGStab's residual peaks stay far below it when it converges).
-constexpr double kDivergence2 = 1e10;
-// Mixed form, stagnation: an FP64 update whose true ||b - A x||^2 is above kStall2 times the last
-// one's (the norm fell by less than 10%), kStallUpdates times in a row.
-constexpr double kStall2 = 0.81;
-constexpr int kStallUpdates = 3;
-
 // Mixed form, after K_XR: the reliable-update test fused with K_P. The FP32 residual triggers an
 // FP64 update when it has dropped by delta since the last one (or looks converged, or the budget
 // is spent). Without an update this kernel is K_P (stop tests, beta, p update) and clears the IF
@@ -1622,7 +1614,10 @@ cudaLaunchConfig_t small_config(int blocks, int threads, size_t smem, bool clust
 }
 
 using SmallKernel = void (*)(const SmallArgs);
-SmallKernel small_kernel(bool merged, bool cluster) {
+SmallKernel small_kernel(bool merged, bool cluster, bool mix) {
+    if (mix)
+        return merged ? (cluster ? k_small_mix<true, true> : k_small_mix<true, false>)
+                      : (cluster ? k_small_mix<false, true> : k_small_mix<false, false>);
     return merged ? (cluster ? k_small<true, true> : k_small<true, false>)
                   : (cluster ? k_small<false, true> : k_small<false, false>);
 }
@@ -1633,6 +1628,11 @@ SmallKernel small_kernel(bool merged, bool cluster) {
 // SM grows; the line lies where it is about 1.5x, so that the loop of a system of tens of thousands of
 // rows and more keeps its summation order and its 4 or 5 launches an iteration.
 constexpr int kSmallRows = 40000;
+// The mixed form's line: its counts, and with them the solution within its tolerance, move more with the
+// order of the sums (2D stencils at rtol 1e-12: by 3e-10 up to 125^2, by 1e-9 at 200^2, as two runs of the
+// graph loop with other sums would), so larger systems keep the loop they had.
+constexpr int kSmallMixRows = 16384;
+bool small_mix(const Solver *s) { return s->small_grid > 0 && s->n <= kSmallMixRows; }
 
 hhp_status ensure_small(Solver *s) {
     if (s->small_grid >= 0) return HHP_OK;
@@ -1656,7 +1656,8 @@ hhp_status ensure_small(Solver *s) {
     while (threads < rows) threads *= 2;
     const size_t smem = static_cast<size_t>(k) * static_cast<size_t>(rows) * 12;
     if (k > kSmallMaxK || threads > kSmallThreads || smem + sizeof(SmallShared) + 1024 > A->ctx->smem_optin) return HHP_OK;
-    for (const SmallKernel kern : {small_kernel(true, cluster), small_kernel(false, cluster)}) {
+    for (const SmallKernel kern : {small_kernel(true, cluster, false), small_kernel(false, cluster, false),
+                                   small_kernel(true, cluster, true), small_kernel(false, cluster, true)}) {
         HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         int fit = 0;  // every block has to be resident
         if (cluster) {
@@ -1685,11 +1686,11 @@ hhp_status ensure_small(Solver *s) {
     return HHP_OK;
 }
 
-hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
+hhp_status launch_small(Solver *s, cudaStream_t st, bool merged, bool mix = false) {
     hhp_mat *A = s->A;
     const PlanDev &p = A->plan64;
     SmallArgs a;
-    a.sc = s->sc;
+    a.sc = mix ? s->sc32 : s->sc;
     a.slice_ptr = p.slice_ptr;
     a.pos_row = p.has_perm ? p.pos_row : nullptr;
     a.pos_len = p.pos_len;
@@ -1708,6 +1709,8 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
     a.S = s->S;
     a.B = s->B;
     a.RV = s->RV;
+    a.P32 = s->P32;
+    a.RV32 = reinterpret_cast<float2 *>(s->RV);  // the FP64 form's, not in use meanwhile
     a.rec = s->small_rec;
     a.arrived = s->small_arrived;
     a.hist = s->hist;
@@ -1715,10 +1718,11 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged) {
     a.dev_err = A->ctx->dev_err;
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg =
-        small_config(s->small_grid, s->small_threads, static_cast<size_t>(s->small_k) * static_cast<size_t>(s->small_rows) * 12,
+        small_config(s->small_grid, s->small_threads,
+                     static_cast<size_t>(s->small_k) * static_cast<size_t>(s->small_rows) * (mix ? 8 : 12),
                      s->small_cluster, st, attr);
     if (!s->small_cluster) HHP_CUDA(cudaMemsetAsync(s->small_arrived, 0, sizeof(unsigned), st));
-    HHP_CUDA(cudaLaunchKernelEx(&cfg, small_kernel(merged, s->small_cluster), a));
+    HHP_CUDA(cudaLaunchKernelEx(&cfg, small_kernel(merged, s->small_cluster, mix), a));
     return HHP_OK;
 }
 
@@ -1873,14 +1877,19 @@ hhp_status build_g64(Solver *s, bool merged, bool ilu = false) {
 hhp_status build_gmix(Solver *s, bool merged) {
     hhp_mat *A = s->A;
     cudaStream_t st = A->ctx->stream;
+    const bool small = small_mix(s);
     HHP_TRY(ensure_plan(A, false));
-    HHP_TRY(ensure_plan(A, true));
+    if (!small) HHP_TRY(ensure_plan(A, true));
     const int nu4 = s->n_pad / 4;
     HHP_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
     hhp_status rc = HHP_OK;
     do {
         if (cudaMemcpyAsync(s->sc32, s->h_sc32, kCtlBytes, cudaMemcpyHostToDevice, st) != cudaSuccess) {
             rc = HHP_ERR_CUDA;
+            break;
+        }
+        if (small) {  // one kernel for the whole pass
+            rc = launch_small(s, st, merged, true);
             break;
         }
         rc = launch_x0check(s, st);
@@ -1913,7 +1922,7 @@ hhp_status build_gmix(Solver *s, bool merged) {
     s->gmix_kernels_pro = 4;
     s->gmix_kernels_epi = 3;
     // launch_spmv* counted their captured launches; graph launches are counted when executed.
-    A->ctx->kernel_launches -= 2 + 3 * s->unroll;
+    if (!small) A->ctx->kernel_launches -= 2 + 3 * s->unroll;
     return HHP_OK;
 }
 
@@ -1925,6 +1934,12 @@ hhp_status build_gmix(Solver *s, bool merged) {
 hhp_status run_direct_mix(Solver *s, bool merged) {
     hhp_mat *A = s->A;
     cudaStream_t st = A->ctx->stream;
+    if (small_mix(s)) {
+        HHP_CUDA(cudaMemcpyAsync(s->sc32, s->h_sc32, kCtlBytes, cudaMemcpyHostToDevice, st));
+        HHP_TRY(launch_small(s, st, merged, true));
+        A->ctx->kernel_launches += 1;
+        return HHP_OK;
+    }
     HHP_TRY(ensure_plan(A, false));
     HHP_TRY(ensure_plan(A, true));
     const int nu4 = s->n_pad / 4;
@@ -2166,6 +2181,7 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
     } else {
         const bool merged32 = o->loop != HHP_LOOP_CLASSIC;
         const bool use_graph = env_int("HHP_SOLVE_GRAPH", 1) != 0;
+        HHP_TRY(ensure_small(s));
         cudaGraphExec_t &gm = merged32 ? s->gmixm : s->gmix;
         if (use_graph && !gm) HHP_TRY(build_gmix(s, merged32));
         DevScal &h32 = *s->h_sc32;
@@ -2186,8 +2202,11 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
             HHP_TRY(readback(s->h_sc32, s->sc32));
             // 4 (merged) or 5 kernels per iteration, 3 more per FP64 update (the IF body)
             if (use_graph)
-                ctx->kernel_launches += s->gmix_kernels_pro + s->gmix_kernels_epi +
-                                        (merged32 ? 4LL : 5LL) * s->unroll * h32.bodies + 3LL * (h32.updates - upd0);
+                ctx->kernel_launches += small_mix(s)
+                                            ? 1
+                                            : s->gmix_kernels_pro + s->gmix_kernels_epi +
+                                                  (merged32 ? 4LL : 5LL) * s->unroll * h32.bodies +
+                                                  3LL * (h32.updates - upd0);
             // an inner breakdown or divergence after some progress restarts the FP32 recurrences
             // once from the last FP64 iterate (its true residual becomes the new shadow
             // residual); a second one hands the solve to FP64 below

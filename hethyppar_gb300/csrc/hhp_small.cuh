@@ -51,6 +51,8 @@ struct SmallArgs {
     double *X, *P, *S;
     const double *B;
     double2 *RV;              // {r, v}
+    float *P32;               // mixed form: p, {r, v}
+    float2 *RV32;
     double *rec;              // 2 sets of kSmallQ * grid partial sums, used in turn
     unsigned *arrived;        // blocks that have arrived, over all exchanges (zero at the launch)
     double *hist;
@@ -161,6 +163,35 @@ __device__ __forceinline__ bool exchange(const SmallArgs &a, SmallShared &sh, co
     }
 }
 
+// Sum over a row's entries, in order, of val * get(col): eight gathers in flight, as many steps as the
+// warp's longest row has, kmax (a multiply-add that no lane needs still takes the FP64 pipe's slot).
+template <typename T, typename G>
+__device__ __forceinline__ T small_row_sum(const T *sv, const int *sc, int ld, int len, int kmax, G get) {
+    T acc = T(0);
+    auto steps = [&](auto n, int k) {
+        constexpr int N = decltype(n)::value;
+        T g[N];
+#pragma unroll
+        for (int u = 0; u < N; ++u) g[u] = k + u < len ? get(sc[(k + u) * ld]) : T(0);
+#pragma unroll
+        for (int u = 0; u < N; ++u)
+            if (k + u < len) acc = tfma(sv[(k + u) * ld], g[u], acc);
+    };
+    int k = 0;
+    for (; k + 8 <= kmax; k += 8) steps(std::integral_constant<int, 8>(), k);
+    switch (kmax - k) {
+        case 1: steps(std::integral_constant<int, 1>(), k); break;
+        case 2: steps(std::integral_constant<int, 2>(), k); break;
+        case 3: steps(std::integral_constant<int, 3>(), k); break;
+        case 4: steps(std::integral_constant<int, 4>(), k); break;
+        case 5: steps(std::integral_constant<int, 5>(), k); break;
+        case 6: steps(std::integral_constant<int, 6>(), k); break;
+        case 7: steps(std::integral_constant<int, 7>(), k); break;
+        default: break;
+    }
+    return acc;
+}
+
 template <bool MERGED, bool CLUSTER>
 __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constant__ SmallArgs a) {
     extern __shared__ double s_mat[];  // val[K][rows], then col[K][rows]
@@ -203,34 +234,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
         x = a.X[row];
         b = a.B[row];
     }
-    // sum over the row's entries, in order, of val * get(col): eight gathers in flight, as many steps as
-    // the warp's longest row has (a multiply-add that no lane needs still takes the FP64 pipe's slot)
     const int kmax = __reduce_max_sync(0xffffffffu, len);
-    auto row_sum = [&](auto get) {
-        double acc = 0.0;
-        auto steps = [&](auto n, int k) {
-            constexpr int N = decltype(n)::value;
-            double g[N];
-#pragma unroll
-            for (int u = 0; u < N; ++u) g[u] = k + u < len ? get(sc_[(k + u) * ld]) : 0.0;
-#pragma unroll
-            for (int u = 0; u < N; ++u)
-                if (k + u < len) acc = fma(sv[(k + u) * ld], g[u], acc);
-        };
-        int k = 0;
-        for (; k + 8 <= kmax; k += 8) steps(std::integral_constant<int, 8>(), k);
-        switch (kmax - k) {
-            case 1: steps(std::integral_constant<int, 1>(), k); break;
-            case 2: steps(std::integral_constant<int, 2>(), k); break;
-            case 3: steps(std::integral_constant<int, 3>(), k); break;
-            case 4: steps(std::integral_constant<int, 4>(), k); break;
-            case 5: steps(std::integral_constant<int, 5>(), k); break;
-            case 6: steps(std::integral_constant<int, 6>(), k); break;
-            case 7: steps(std::integral_constant<int, 7>(), k); break;
-            default: break;
-        }
-        return acc;
-    };
+    auto row_sum = [&](auto get) { return small_row_sum<double>(sv, sc_, ld, len, kmax, get); };
     const double none[1] = {0.0};
     // r = b - A x, p = r; ||r||^2, ||b||^2 and whether x0 has a nonzero. x0 = 0 means r = b, also where
     // A holds an infinity or a NaN (the loop finds it): formed again then.
@@ -428,6 +433,288 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
         sc->bodies = 0;
         sc->arrivals = 0;
         sc->rr_last = rr;
+        sc->true_rr = true_rr;
+    }
+}
+
+// Growth of the FP32 recursive ||r||^2 over the last true ||b - A x||^2 taken as divergence
+// (a factor 1e5 in the norm: BiCGStab's residual peaks stay far below it when it converges).
+constexpr double kDivergence2 = 1e10;
+// Mixed form, stagnation: an FP64 update whose true ||b - A x||^2 is above kStall2 times the last
+// one's (the norm fell by less than 10%), kStallUpdates times in a row.
+constexpr double kStall2 = 0.81;
+constexpr int kStallUpdates = 3;
+
+// The mixed form of a small system (see K_MIX_INIT to K_MIX_FINAL): the FP32 recurrences as in k_small,
+// the FP64 iterate and residual per row in the thread's registers. 5-point stencils, us an inner iteration
+// against the graph loop: 100^2 11.9 / 22.7, 125^2 11.2 / 23.2; whole solves: 4,291 and 10,033 rows of 17
+// entries 364 / 936 and 396 / 944 us, 16^3 7-point 537 / 1651 us.
+// An FP64 update is two exchanges (every x visible; the sums) and a product with the FP64 values from
+// L2, a few times per solve. t = A s always forms s from r and v: an FP32 multiply-add an entry costs
+// next to nothing beside an exchange.
+template <bool MERGED, bool CLUSTER>
+__global__ void __launch_bounds__(kSmallThreads, 1) k_small_mix(const __grid_constant__ SmallArgs a) {
+    extern __shared__ double s_mat[];  // float val[K][rows], then col[K][rows]
+    __shared__ SmallShared sh;
+    const int t = threadIdx.x, pos = blockIdx.x * a.rows + t;
+    const bool own = t < a.rows && pos < a.n, lead = blockIdx.x == 0 && t == 0;
+    const int row = own && a.pos_row ? a.pos_row[pos] : pos;
+    float *sv = reinterpret_cast<float *>(s_mat) + t;
+    int *sc_ = reinterpret_cast<int *>(reinterpret_cast<float *>(s_mat) + a.K * a.rows) + t;
+    const int ld = a.rows;
+    DevScal *sc = a.sc;
+    const int restart = sc->restart, maxit = sc->maxit;
+    const double rtol2 = sc->rtol2, inner2 = sc->inner_rtol2, thr2_in = sc->thr2, rr0_in = sc->rr0, bb_in = sc->bb;
+    const int it0 = restart ? sc->iter : 0;
+    unsigned e = 0;
+    int iter = it0, updates = restart ? sc->updates : 0, stalls = 0, status = ST_RUNNING, len = 0, mask = 0;
+    long long base = 0;
+    double x = 0.0, b = 0.0;
+    float d = 0.f, r = 0.f, p = 0.f, v = 0.f, s = 0.f, tv = 0.f;
+    if (own) {
+        base = a.uni ? static_cast<long long>(pos / a.H) * a.nd * a.H + pos % a.H : a.slice_ptr[pos / a.H] + pos % a.H;
+        mask = a.pos_len[pos];
+        if (a.uni) {
+            for (int k = 0; k < a.nd; ++k)
+                if (mask >> k & 1) {
+                    sv[len * ld] = static_cast<float>(a.sval[base + static_cast<long long>(k) * a.H]);
+                    sc_[len * ld] = row + a.doff[k];
+                    ++len;
+                }
+        } else {
+            for (int k = 0; k < mask; ++k) {
+                const long long q = base + static_cast<long long>(k) * a.H;
+                sv[k * ld] = static_cast<float>(a.sval[q]);
+                sc_[k * ld] = a.scol16 ? row + a.scol16[q] : a.scol[q];
+            }
+            len = mask;
+        }
+        x = a.X[row];
+        b = a.B[row];
+    }
+    const int kmax = __reduce_max_sync(0xffffffffu, len);
+    auto row_sum = [&](auto get) { return small_row_sum<float>(sv, sc_, ld, len, kmax, get); };
+    // b - A x of this row in FP64 (every block's x is in a.X)
+    auto residual = [&] {
+        double acc = 0.0;
+        if (a.uni) {
+            int j = 0;
+            for (int k = 0; k < a.nd; ++k)
+                if (mask >> k & 1)
+                    acc = fma(a.sval[base + static_cast<long long>(k) * a.H], __ldcg(a.X + sc_[j++ * ld]), acc);
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < len; ++k)
+                acc = fma(a.sval[base + static_cast<long long>(k) * a.H], __ldcg(a.X + sc_[k * ld]), acc);
+        }
+        return b - acc;
+    };
+    const double none[1] = {0.0};
+    auto publish = [&] {  // r and p, for the other rows after the next exchange
+        if (own) {
+            a.RV32[row].x = r;
+            a.P32[row] = p;
+        }
+    };
+    double rd = residual();
+    r = static_cast<float>(rd);
+    p = r;
+    publish();
+    const double di[4] = {own ? rd * rd : 0.0, own ? b * b : 0.0, own && x != 0.0 ? 1.0 : 0.0,
+                          static_cast<double>(r) * r};
+    bool good = exchange<4, CLUSTER>(a, sh, di, e);
+    double rd2 = sh.tot[0], rho = sh.tot[3], alpha = 1.0, omega = 1.0;
+    const double bb = restart ? bb_in : sh.tot[1], thr2 = restart ? thr2_in : rtol2 * bb;
+    if (good && !isfinite(rd2) && sh.tot[2] == 0.0) {  // x0 = 0: r = b whatever A holds (see k_small)
+        rd2 = sh.tot[1];
+        r = static_cast<float>(b);
+        p = r;
+        publish();
+        const double dr[1] = {static_cast<double>(r) * r};
+        good = exchange<1, CLUSTER>(a, sh, dr, e);
+        rho = sh.tot[0];
+    }
+    const float r0 = r;
+    double true_rr = rd2, rr_max = rd2, rr_last = rd2;
+    // the stop tests of K_MIX_INIT, then of K_P's first run
+    if (rd2 <= rtol2 * bb) {
+        status = ST_CONVERGED;
+    } else if (!isfinite(rd2)) {
+        status = ST_BREAKDOWN;
+    } else {
+        double beta;
+        status = step_p(ST_RUNNING, iter, it0, maxit, -1.0, rho, rho, 0.0, 1.0, 1.0, 1.0, false, beta);
+        rr_last = rho;
+    }
+    __syncthreads();  // sh.tot has been read
+    while (status == ST_RUNNING && good) {
+        // v = A p, alpha
+        v = row_sum([&](int c) { return __ldcg(a.P32 + c); });
+        if (own) a.RV32[row].y = v;
+        const double dv[1] = {own ? static_cast<double>(v) * r0 : 0.0};
+        good = exchange<1, CLUSTER>(a, sh, dv, e);
+        if (!good) break;
+        if (t == 0) {
+            const double rv = sh.tot[0], al = rho / rv;
+            sh.mode = finite_nonzero(rv) && isfinite(al);
+            sh.bc[0] = al;
+        }
+        __syncthreads();
+        if (!sh.mode) {
+            status = ST_BREAKDOWN;
+            break;
+        }
+        alpha = sh.bc[0];
+        const float ta = static_cast<float>(alpha);
+        ++iter;
+        // s, t = A s
+        s = fmaf(-ta, v, r);
+        tv = row_sum([&](int c) {
+            const float2 q = __ldcg(a.RV32 + c);
+            return fmaf(-ta, q.y, q.x);
+        });
+        const double sd = s, td = tv;
+        // what: 0 nothing (the pass ends), 1 d, r and p, 2 an FP64 update
+        if constexpr (MERGED) {
+            const double ds[5] = {own ? td * sd : 0.0, own ? td * td : 0.0, own ? td * r0 : 0.0, own ? sd * sd : 0.0,
+                                  own ? sd * r0 : 0.0};
+            good = exchange<5, CLUSTER>(a, sh, ds, e);
+            if (!good) break;
+            if (t == 0) {  // the step of K_XRP_RU
+                const double ts = sh.tot[0], tt = sh.tot[1], r0t = sh.tot[2], ss = sh.tot[3], r0s = sh.tot[4];
+                const double om = ts / tt, rr = fmax(ss - om * ts, 0.0);
+                int what = 0;
+                sh.bc[0] = om;
+                sh.bc[2] = rr;
+                if (finite_nonzero(tt) && isfinite(om) && isfinite(rr) && !(rr > kDivergence2 * true_rr)) {
+                    if (rr <= thr2 || rr < inner2 * rr_max || iter >= maxit) {
+                        what = 2;
+                    } else {
+                        const double rho_new = r0s - om * r0t;
+                        if (finite_nonzero(rho_new)) {
+                            sh.bc[1] = (rho_new / rho) * (alpha / om);
+                            sh.bc[3] = rho_new;
+                            what = 1;
+                        }
+                    }
+                    if (lead && iter - 1 < a.hist_cap) a.hist[iter - 1] = rr;
+                }
+                sh.mode = what;
+            }
+            __syncthreads();
+        } else {
+            const double ds[2] = {own ? td * sd : 0.0, own ? td * td : 0.0};
+            good = exchange<2, CLUSTER>(a, sh, ds, e);
+            if (!good) break;
+            if (t == 0) {  // the step of K_XR
+                const double om = sh.tot[0] / sh.tot[1];
+                sh.mode = finite_nonzero(sh.tot[1]) && isfinite(om);
+                sh.bc[0] = om;
+            }
+            __syncthreads();
+            if (!sh.mode) {
+                status = ST_BREAKDOWN;
+                break;
+            }
+            const double rn = fmaf(-static_cast<float>(sh.bc[0]), tv, s);
+            const double d2[2] = {own ? rn * r0 : 0.0, own ? rn * rn : 0.0};
+            good = exchange<2, CLUSTER>(a, sh, d2, e);
+            if (!good) break;
+            if (t == 0) {  // the step of K_P_RU
+                const double rho_new = sh.tot[0], rr = sh.tot[1];
+                int what = 0;
+                sh.bc[2] = rr;
+                if (isfinite(rr) && !(rr > kDivergence2 * true_rr)) {
+                    if (rr <= thr2 || rr < inner2 * rr_max || iter >= maxit) {
+                        what = 2;
+                    } else if (finite_nonzero(rho_new)) {
+                        sh.bc[1] = (rho_new / rho) * (alpha / sh.bc[0]);
+                        sh.bc[3] = rho_new;
+                        what = 1;
+                    }
+                    if (lead && iter - 1 < a.hist_cap) a.hist[iter - 1] = rr;
+                }
+                sh.mode = what;
+            }
+            __syncthreads();
+        }
+        const int what = sh.mode;
+        if (what == 0) {  // d is dropped: x stays as of the last update
+            status = ST_BREAKDOWN;
+            break;
+        }
+        omega = sh.bc[0];
+        const float tw = static_cast<float>(omega);
+        d = fmaf(tw, s, fmaf(ta, p, d));
+        if (what == 1) {
+            const float tb = static_cast<float>(sh.bc[1]);
+            rho = sh.bc[3];
+            rr_last = sh.bc[2];
+            rr_max = fmax(rr_max, rr_last);
+            r = fmaf(-tw, tv, s);
+            p = fmaf(tb, fmaf(-tw, v, p), r);
+        } else {
+            // x += d and the true residual; its FP32 value replaces r (K_RU_APPLY, then K_P)
+            x += static_cast<double>(d);
+            d = 0.f;
+            if (own) a.X[row] = x;
+            good = exchange<0, CLUSTER>(a, sh, none, e);
+            if (!good) break;
+            rd = residual();
+            r = static_cast<float>(rd);
+            const double du[3] = {own ? rd * rd : 0.0, own ? static_cast<double>(r) * r0 : 0.0,
+                                  own ? static_cast<double>(r) * r : 0.0};
+            good = exchange<3, CLUSTER>(a, sh, du, e);
+            if (!good) break;
+            rd2 = sh.tot[0];
+            const double rho_new = sh.tot[1], rr = sh.tot[2];
+            rr_max = rd2;
+            ++updates;
+            stalls = rd2 > kStall2 * true_rr ? stalls + 1 : 0;
+            true_rr = rd2;
+            if (rd2 <= thr2) status = ST_CONVERGED;
+            else if (!isfinite(rd2) || stalls >= kStallUpdates) status = ST_BREAKDOWN;
+            else if (iter >= maxit) status = ST_MAXIT;
+            if (status != ST_RUNNING) break;
+            if (lead && iter - 1 < a.hist_cap) a.hist[iter - 1] = rr;
+            rr_last = rr;
+            if (t == 0) {
+                double beta = 0.0;
+                sh.mode = step_p(ST_RUNNING, iter, it0, maxit, -1.0, rho_new, rr, 0.0, rho, alpha, omega, false, beta);
+                sh.bc[1] = beta;
+            }
+            __syncthreads();
+            status = sh.mode;
+            if (status != ST_RUNNING) break;
+            rho = rho_new;
+            p = fmaf(static_cast<float>(sh.bc[1]), fmaf(-tw, v, p), r);
+        }
+        publish();
+        good = exchange<0, CLUSTER>(a, sh, none, e);
+    }
+    // (x holds every folded increment; the one since is zero or, after a breakdown, dropped)
+    if (own) a.X[row] = x;
+    if (good) good = exchange<0, CLUSTER>(a, sh, none, e);
+    if (good) {
+        const double res = residual();
+        const double df[1] = {own ? res * res : 0.0};
+        good = exchange<1, CLUSTER>(a, sh, df, e);
+        true_rr = sh.tot[0];
+    }
+    if (lead) {
+        sc->status = good ? status : ST_DEVICE_ERROR;
+        sc->rr0 = restart ? rr0_in : bb;
+        sc->bb = bb;
+        sc->thr2 = thr2;
+        sc->thr2_rec = -1.0;
+        sc->iter = iter;
+        sc->iter_start = it0;
+        sc->updates = updates;
+        sc->stalls = stalls;
+        sc->bodies = 0;
+        sc->arrivals = 0;
+        sc->ru_flag = 0;
+        sc->rr_last = rr_last;
         sc->true_rr = true_rr;
     }
 }
