@@ -11,8 +11,9 @@
 namespace hhp {
 
 // Device error codes for the context's error word. The only waits in this library are the grid
-// barriers between dependency levels inside the ILU(0) kernels (cooperative launches, so every
-// block is resident); each is bounded, and one that runs out sets DEV_ERR_TIMEOUT. SpMV launches,
+// barriers between dependency levels inside the ILU(0) kernels and the exchanges of the one-kernel
+// solves (cooperative or one-cluster launches, so every block is resident); each on memory is
+// bounded, and one that runs out sets DEV_ERR_TIMEOUT. SpMV launches,
 // the ILU kernels and the solve loop check the word, so every later launch stops and the solve
 // returns HHP_ERR_TIMEOUT. (The SpMV's long-row combine is a last-arriver atomic count, not a
 // wait; every other ordering is a kernel boundary.)

@@ -27,6 +27,7 @@
 // partials in a fixed order (so every block gets the same scalar, bit for bit, and runs are
 // reproducible). No host synchronisation inside the loop: kernels read the scalars from device
 // memory and the kernel with the stop tests ends the WHILE loop with cudaGraphSetConditional.
+// Small systems run either schedule as one kernel instead (hhp_small.cuh).
 #include <algorithm>
 #include <cmath>
 #include <cstddef>
@@ -1622,8 +1623,9 @@ SmallKernel small_kernel(bool merged, bool cluster, bool mix) {
                   : (cluster ? k_small<false, true> : k_small<false, false>);
 }
 
-// Decides once per matrix whether its FP64 loop runs as k_small, and lays out what that needs: at most
-// kSmallRows rows, none of them cut into chunks (a row is one thread's), of at most kSmallMaxK entries, and the blocks' entries in shared memory. The gain over the graph loop falls with
+// Decides once per matrix whether its loop runs as k_small (FP64) and k_small_mix, and lays out what that needs: at most
+// kSmallRows rows, none of them cut into chunks (a row is one thread's), of at most kSmallMaxK entries,
+// and the blocks' entries in shared memory. The gain over the graph loop falls with
 // the size (5-point stencils: 1.9x at 8,100 rows, 1.7x at 16,384, 1.34x at 62,500), as the FP64 work per
 // SM grows; the line lies where it is about 1.5x, so that the loop of a system of tens of thousands of
 // rows and more keeps its summation order and its 4 or 5 launches an iteration.

@@ -1,4 +1,4 @@
-// hhp_small.cuh -- the FP64 BiCGStab loop of a small system as one cooperative kernel.
+// hhp_small.cuh -- the BiCGStab solve of a small system as one kernel, in FP64 and in the mixed form.
 //
 // 5-point stencils, us an iteration against the graph loop: 32^2 7.9 / 19.4, 64^2 9.1 / 19.7, 128^2
 // 11.7 / 20.1 (classic 64^2 10.1 / 25.0); 17 entries per row: 4,000 rows 14.0 / 27.5, 20,000 rows
@@ -21,8 +21,8 @@
 // pushed into every block's shared memory and the hardware's cluster barrier (556 cycles at 16
 // blocks). Above that the FP64 work of 16 SMs outweighs the cheaper exchange: the grid is launched
 // cooperatively (all blocks resident) and an exchange is records in L2 and an arrival count that every
-// block polls (1.2 us; polling all blocks' records instead took 3.3 us at 152 blocks). Every such wait is bounded: one that runs out sets the
-// context's error word and the block leaves, as the others then do. All blocks add the same numbers in
+// block polls (1.2 us; polling all blocks' records instead took 3.3 us at 152 blocks). Every such wait
+// is bounded: one that runs out sets the context's error word and the block leaves, as the others then do. All blocks add the same numbers in
 // the same order, so they compute the same scalars bit for bit and take the same branches.
 #pragma once
 

@@ -82,7 +82,7 @@ typedef enum {
  * products reach a lower true residual). Fixed-iteration runs always use CLASSIC. ILU(0) adds its
  * two applications to either schedule (MERGED: 8 kernels per iteration, CLASSIC: 9). The FP32
  * inner loop of the mixed form follows the same choice (MERGED: its kernel with the x and r
- * updates also takes the reliable-update test). */
+ * updates also takes the reliable-update test). Small systems run either order as one kernel. */
 typedef enum { HHP_LOOP_AUTO = 0, HHP_LOOP_MERGED = 1, HHP_LOOP_CLASSIC = 2 } hhp_loop;
 
 typedef struct {
