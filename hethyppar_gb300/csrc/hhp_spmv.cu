@@ -607,7 +607,14 @@ __device__ __forceinline__ T ld_value(const T *p) {
 //  * all K values and entries of x are requested at once. A lane's R rows take two passes of R/2, so
 //    that 2 K R/2 words fit the registers of the occupancy that HBM latency needs (32 warps per SM
 //    FP32, 40 FP64); the second pass finds its half of every sector of the value stream in L1. One
-//    pass at that occupancy spills, and with fewer warps it is slower (FP32, 160^3: 37 us).
+//    pass at that occupancy spills, and with fewer warps it is slower (FP32, 160^3: 37 us);
+//  * FP32 rows of 7 take both passes' values with one 16-byte load a diagonal, where the entries of x alone
+//    come in two passes (64 registers): half the L1's work on the stream, and no second touch that
+//    streaming loads may find gone (160^3 mixed 102.7 -> 97.2 us an iteration, 125^3 58.0 -> 53.9). Rows of
+//    5 do not gain (2048^2: 20.8 -> 22.6 us);
+//  * beside the main diagonal, x[i - 1] and x[i + 1] share its words: a scalar load each per pair of rows
+//    instead of two (FP32 160^3 28.7 -> 26.7 us, 100^3 9.3 -> 8.3, 2048^2 22.0 -> 20.8). With streaming
+//    loads in two passes it lost (160^3 mixed 102.7 -> 110.9): not there.
 // Lanes own the same rows and units as in the general kernel, so the dot products' partial sums are
 // the same too, bit for bit. 160^3 7-point: FP32 32.8 -> 28.4 us (the mixed solve 119.8 -> 108.7 us
 // an iteration), FP64 60.2 -> 58.5 us; 256^2 5-point FP64 6.2 -> 4.2 us (23.0 -> 21.7 us a solve iteration).
@@ -616,12 +623,15 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
     constexpr int H = 32 * R, N = R / 2;  // N rows per lane and pass
     using VN = typename Vec<VT, N>::V;
     using VV = typename Vec<VT, R>::V;
+    constexpr bool WHOLE = N == 2 && K == 7;  // both passes' values with one 16-byte load each
     constexpr bool W1 = EP == EP_DOT1 || EP == EP_DOT2 || EP == EP_DOT3 || EP == EP_RESID;
     __shared__ double red[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int gw = blockIdx.x * nw + warp, W = gridDim.x * nw;
     const int err = __ldcg(a.err), gate = a.gate ? __ldcg(a.gate) : 1, stop = a.stop ? __ldcg(a.stop) : 0;
     const bool skip = err != DEV_OK || gate == 0 || stop != 0;
+    // diagonals -1, 0, 1 in the middle: the neighbours share the main diagonal's words
+    const bool mid = N == 2 && (WHOLE || !ONCE) && a.x_vec && a.doff[K / 2] == 0 && a.doff[K / 2 - 1] == -1 && a.doff[K / 2 + 1] == 1;
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int u = gw; u < a.n_slices; u += W) {
         const int q0 = u * H + lane * R;
@@ -632,15 +642,31 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
         // every diagonal of every row of the slice lies inside x
         const bool safe = u * H + a.doff[0] >= 0 && u * H + H + a.doff[K - 1] <= a.n;
         VT acc[R];
+        VV v4[WHOLE ? K : 1];
+        if constexpr (WHOLE) {
+#pragma unroll
+            for (int k = 0; k < K; ++k) v4[k] = ld_value<ONCE>(reinterpret_cast<const VV *>(vp + k * H));
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            VN v[K];
+            VN v[WHOLE ? 1 : K];
             VT xv[K][N];
+            if constexpr (!WHOLE) {
 #pragma unroll
-            for (int k = 0; k < K; ++k) v[k] = ld_value<ONCE>(reinterpret_cast<const VN *>(vp + k * H + N * h));
+                for (int k = 0; k < K; ++k) v[k] = ld_value<ONCE>(reinterpret_cast<const VN *>(vp + k * H + N * h));
+            }
             if (safe) {
 #pragma unroll
-                for (int k = 0; k < K; ++k) load_run<VT, N>(xv[k], a.x, q0 + N * h + a.doff[k], a.doff[k], a.x_vec);
+                for (int k = 0; k < K; ++k)
+                    if (!mid || (k != K / 2 - 1 && k != K / 2 + 1))
+                        load_run<VT, N>(xv[k], a.x, q0 + N * h + a.doff[k], a.doff[k], a.x_vec);
+                if (mid) {
+                    const VT *xc = a.x + q0 + N * h;
+                    xv[K / 2 - 1][0] = __ldg(xc - 1);
+                    xv[K / 2 - 1][N - 1] = xv[K / 2][0];
+                    xv[K / 2 + 1][0] = xv[K / 2][N - 1];
+                    xv[K / 2 + 1][N - 1] = __ldg(xc + N);
+                }
             } else {
 #pragma unroll
                 for (int k = 0; k < K; ++k)
@@ -656,7 +682,9 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
 #pragma unroll
                 for (int t = 0; t < N; ++t)
                     if ((mw >> (8 * (N * h + t) + k)) & 1)
-                        acc[N * h + t] = vfma(comp<VN, VT>(v[k], t), xv[k][t], acc[N * h + t]);
+                        acc[N * h + t] = vfma(WHOLE ? comp<VV, VT>(v4[WHOLE ? k : 0], N * h + t)
+                                                    : comp<VN, VT>(v[WHOLE ? 0 : k], t),
+                                              xv[k][t], acc[N * h + t]);
         }
         VT w1v[R], w2v[R];
         VV z1 = VV(), z2 = VV();

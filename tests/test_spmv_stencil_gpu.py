@@ -89,3 +89,33 @@ def test_values_refresh_and_dropped_csr(ctx):
     x2, r2 = bicgstab(ctx, A, s.b, rtol=1e-10)
     assert np.array_equal(x, x2) and r.iters == r2.iters
     A.close()
+
+
+@pytest.mark.parametrize("offsets", [(0, 1, 2, 3, 4), (-3, -2, -1, 0, 1), (-64, -2, 0, 2, 64), (-9, -1, 0, 1, 2),
+                                     (-65, -1, 0, 1, 66), (-100, -7, -1, 0, 1, 7, 100), (-96, -8, -2, 0, 3, 8, 96),
+                                     (-3, -2, -1, 0, 1, 2, 3), (-5, -4, -3, -1, 0, 1, 2)])
+def test_middle_diagonals(ctx, offsets):
+    """Diagonals beside the main one share its words of x; other sets of 5 and 7 do not."""
+    n = 128 * 70 + 37
+    rng = np.random.default_rng(n)
+    cols = np.arange(n)[:, None] + np.array(offsets)
+    keep = (cols >= 0) & (cols < n) & (rng.random(cols.shape) > 0.03)
+    rp = np.concatenate([[0], np.cumsum(keep.sum(1))]).astype(np.int32)
+    col = cols[keep].astype(np.int32)
+    val, x = rng.standard_normal(col.size), rng.standard_normal(n)
+    A = Matrix.from_csr(ctx, rp, col, val, shape=(n, n))
+    assert np.array_equal(A.spmv(x), orc.spmv(rp, col, val, x, fma=True))
+    x32, v32 = x.astype(np.float32), val.astype(np.float32)
+    exact = orc.spmv(rp, col, v32.astype(np.float64), x32.astype(np.float64))
+    bound = 8 * 2.0 ** -24 * orc.spmv(rp, col, np.abs(v32).astype(np.float64), np.abs(x32).astype(np.float64))
+    first = None
+    for off in range(4):
+        xd = torch.zeros(n + 4, dtype=torch.float32, device="cuda")[off:off + n]
+        xd.copy_(dev(x32, torch.float32))
+        y = torch.full((n,), float("nan"), dtype=torch.float32, device="cuda")
+        A.spmv_f32_dev(xd, y)
+        got = y.cpu().numpy()
+        assert np.all(np.abs(got - exact) <= bound)
+        first = got if first is None else first
+        assert np.array_equal(got, first)
+    A.close()
