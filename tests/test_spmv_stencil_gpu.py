@@ -119,3 +119,18 @@ def test_middle_diagonals(ctx, offsets):
         first = got if first is None else first
         assert np.array_equal(got, first)
     A.close()
+
+
+@pytest.mark.parametrize("dims", [(550, 40, 40), (600, 40, 40), (985, 40, 40)])
+def test_loop_kernel_by_size(ctx, dims):
+    """Systems on both sides of the sizes whose loop products take the general kernel: the first iterations
+    of both schedules as the reference's loop has them."""
+    rp, col, val = synth._stencil(dims, 20.0, (1.0, 0.5, 0.25))
+    n = rp.size - 1
+    b = np.random.default_rng(n).standard_normal(n)
+    ref = orc.bicgstab_fixed(rp, col, val, b, np.zeros(n), 3)[0]
+    A = Matrix.from_csr(ctx, rp, col, val)
+    for loop in ("merged", "classic"):
+        x, r = bicgstab(ctx, A, b, rtol=1e-12, maxit=3, loop=loop)
+        assert r.iters == 3 and np.max(np.abs(x - ref)) <= 1e-10 * max(1.0, np.max(np.abs(ref)))
+    A.close()
