@@ -22,8 +22,9 @@
 // blocks). Above that the FP64 work of 16 SMs outweighs the cheaper exchange: the grid is launched
 // cooperatively (all blocks resident) and an exchange is records in L2 and an arrival count that every
 // block polls (1.2 us; polling all blocks' records instead took 3.3 us at 152 blocks). Every such wait
-// is bounded: one that runs out sets the context's error word and the block leaves, as the others then do. All blocks add the same numbers in
-// the same order, so they compute the same scalars bit for bit and take the same branches.
+// is bounded: one that runs out sets the context's error word and the block leaves, as the others then
+// do. All blocks add the same numbers in the same order, so they compute the same scalars bit for bit and
+// take the same branches.
 #pragma once
 
 constexpr int kSmallThreads = 512;

@@ -1,6 +1,6 @@
-"""New values reach every layout through the staged re-layout: rows of one length up to the slice limit (one
-chunk and several per warp, lengths that share banks), ragged and empty rows, rows that long rows or the
-sorting take out of order; FP64, FP32 before and after its first use, and the transpose."""
+"""New values reach every layout: rows of one length up to the slice limit, ragged and empty rows, rows
+that long rows or the sorting take out of order; FP64, FP32 before and after its first use, and the
+transpose."""
 import numpy as np
 import pytest
 
