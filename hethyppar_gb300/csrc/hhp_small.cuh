@@ -86,12 +86,18 @@ __device__ __forceinline__ void block_tree(SmallShared &sh, const double (&v)[NQ
     }
 }
 
+// The first exchange writes other blocks' shared memory, which may only be done once every block of the
+// cluster runs. cluster_start() says so of this block, cluster_started() waits for all; between the two a
+// kernel stages its matrix, so the wait costs nothing. (Not .aligned: lanes may arrive apart.)
+__device__ __forceinline__ void cluster_start() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_started() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // One exchange of NQ sums (NQ = 0: a barrier), number e = 1, 2, ... of the launch; the sums in
-// sh.tot. The blocks' earlier global stores are visible to every block after it. The buffers of e are
+// sh.tot. (CLUSTER: after cluster_started().) The blocks' earlier global stores are visible to every block after it. The buffers of e are
 // written again at e + 2, which a block reaches only after every block has arrived at e + 1, that is
 // has read e's. Returns false when the wait ran out (uniform across the block).
 template <int NQ, bool CLUSTER>
@@ -200,6 +206,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
     const int t = threadIdx.x, pos = blockIdx.x * a.rows + t;
     const bool own = t < a.rows && pos < a.n, lead = blockIdx.x == 0 && t == 0;
     const int row = own && a.pos_row ? a.pos_row[pos] : pos;
+    if constexpr (CLUSTER) cluster_start();
     double *sv = s_mat + t;
     int *sc_ = reinterpret_cast<int *>(s_mat + a.K * a.rows) + t;
     const int ld = a.rows;
@@ -250,6 +257,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small(const __grid_constan
     };
     publish();
     const double di[3] = {own ? r * r : 0.0, own ? b * b : 0.0, own && x != 0.0 ? 1.0 : 0.0};
+    if constexpr (CLUSTER) cluster_started();
     bool good = exchange<3, CLUSTER>(a, sh, di, e);
     double rr = sh.tot[0], alpha = 1.0, omega = 1.0;
     const double bb = sh.tot[1], thr2 = restart ? thr2_in : fixed ? -1.0 : rtol2 * bb;
@@ -460,6 +468,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_mix(const __grid_con
     const int t = threadIdx.x, pos = blockIdx.x * a.rows + t;
     const bool own = t < a.rows && pos < a.n, lead = blockIdx.x == 0 && t == 0;
     const int row = own && a.pos_row ? a.pos_row[pos] : pos;
+    if constexpr (CLUSTER) cluster_start();
     float *sv = reinterpret_cast<float *>(s_mat) + t;
     int *sc_ = reinterpret_cast<int *>(reinterpret_cast<float *>(s_mat) + a.K * a.rows) + t;
     const int ld = a.rows;
@@ -523,6 +532,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_mix(const __grid_con
     publish();
     const double di[4] = {own ? rd * rd : 0.0, own ? b * b : 0.0, own && x != 0.0 ? 1.0 : 0.0,
                           static_cast<double>(r) * r};
+    if constexpr (CLUSTER) cluster_started();
     bool good = exchange<4, CLUSTER>(a, sh, di, e);
     double rd2 = sh.tot[0], rho = sh.tot[3], alpha = 1.0, omega = 1.0;
     const double bb = restart ? bb_in : sh.tot[1], thr2 = restart ? thr2_in : rtol2 * bb;
