@@ -1657,10 +1657,13 @@ hhp_status ensure_small(Solver *s) {
     int threads = 32;  // a power of two (the reduction tree), a row each
     while (threads < rows) threads *= 2;
     const size_t smem = static_cast<size_t>(k) * static_cast<size_t>(rows) * 12;
-    if (k > kSmallMaxK || threads > kSmallThreads || smem + sizeof(SmallShared) + 1024 > A->ctx->smem_optin) return HHP_OK;
+    // The limit belongs to the function on its device: set to what one matrix needs, it would refuse the
+    // launches of an earlier one that needs more. So it is the same for all, whatever a block could ask for.
+    const size_t room = A->ctx->smem_optin - sizeof(SmallShared) - 1024;
+    if (k > kSmallMaxK || threads > kSmallThreads || smem > room) return HHP_OK;
     for (const SmallKernel kern : {small_kernel(true, cluster, false), small_kernel(false, cluster, false),
                                    small_kernel(true, cluster, true), small_kernel(false, cluster, true)}) {
-        HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(room)));
         int fit = 0;  // every block has to be resident
         if (cluster) {
             HHP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
