@@ -254,6 +254,12 @@ hhp_status mat_create_dev(hhp_ctx *ctx, int m, int n, int nnz, hhp_mat **out);  
 hhp_status mat_refresh_derived(hhp_mat *A, bool make32 = true);  // after value changes; make32: FP32 values too
 inline int pad4(int n) { return (n + 3) & ~3; }
 
+// Whether an arrival count has reached `target`. Both are taken modulo 2^32, as a long solve of many
+// blocks passes it, and lie less than 2^31 apart.
+__host__ __device__ inline bool count_reached(unsigned seen, unsigned target) {
+    return static_cast<int>(seen - target) >= 0;
+}
+
 // Kernel tuning knobs (environment overrides read once).
 struct Tuning {
     // ctas_per_sm, spmv_unroll, rpl64: 0 = chosen per matrix at plan time; d16 0: never 16-bit offsets

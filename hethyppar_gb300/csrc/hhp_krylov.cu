@@ -1726,7 +1726,8 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged, bool mix = fals
         small_config(s->small_grid, s->small_threads,
                      static_cast<size_t>(s->small_k) * static_cast<size_t>(s->small_rows) * (mix ? 8 : 12),
                      s->small_cluster, st, attr);
-    if (!s->small_cluster) HHP_CUDA(cudaMemsetAsync(s->small_arrived, 0, sizeof(unsigned), st));
+    static_assert(kSmallCount0 == 0xffffffffu, "set byte by byte");
+    if (!s->small_cluster) HHP_CUDA(cudaMemsetAsync(s->small_arrived, 0xff, sizeof(unsigned), st));
     HHP_CUDA(cudaLaunchKernelEx(&cfg, small_kernel(merged, s->small_cluster, mix), a));
     return HHP_OK;
 }

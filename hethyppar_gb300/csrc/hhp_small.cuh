@@ -37,6 +37,9 @@ constexpr int kSmallCluster = 16;         // blocks of the one-cluster form, at 
 constexpr int kSmallClusterRows = 6144;   // 5-point, 4096 rows: 9.1 against 13.9 us an iteration on the
                                           // whole grid, 8100 rows: 12.3 against 12.4; 17 entries per
                                           // row, 4000 rows: 14.0 against 19.1, 8000 rows: 19.1 against 17.8
+// The count starts one below 2^32: a launch of 152 blocks passes 2^32 every 28 million exchanges, and so
+// every launch does in its first.
+constexpr unsigned kSmallCount0 = 0xffffffffu;
 constexpr int kSmallPolls = 1 << 20;      // reads of the count before giving up (~0.5 us each)
 
 struct SmallArgs {
@@ -55,7 +58,7 @@ struct SmallArgs {
     float *P32;               // mixed form: p, {r, v}
     float2 *RV32;
     double *rec;              // 2 sets of kSmallQ * grid partial sums, used in turn
-    unsigned *arrived;        // blocks that have arrived, over all exchanges (zero at the launch)
+    unsigned *arrived;        // blocks that have arrived, over all exchanges, from kSmallCount0
     double *hist;
     int hist_cap;
     int *dev_err;
@@ -141,11 +144,14 @@ __device__ __forceinline__ bool exchange(const SmallArgs &a, SmallShared &sh, co
         if (t == 0) {
             // the block's stores (ordered before this by the barrier) before its arrival
             asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(a.arrived) : "memory");
-            const unsigned target = e * static_cast<unsigned>(G);
-            unsigned seen = 0;
-            for (int i = 0; i < kSmallPolls && seen < target; ++i)
+            const unsigned target = kSmallCount0 + e * static_cast<unsigned>(G);
+            bool all = false;
+            for (int i = 0; i < kSmallPolls && !all; ++i) {
+                unsigned seen;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.arrived) : "memory");
-            sh.ok = seen >= target;
+                all = count_reached(seen, target);
+            }
+            sh.ok = all;
         }
         __syncthreads();
         if (!sh.ok) {
