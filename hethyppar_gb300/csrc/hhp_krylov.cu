@@ -1720,6 +1720,7 @@ hhp_status launch_small(Solver *s, cudaStream_t st, bool merged, bool mix = fals
     a.arrived = s->small_arrived;
     a.hist = s->hist;
     a.hist_cap = s->hist_cap;
+    a.polls = env_int("HHP_SMALL_POLLS", kSmallPolls);
     a.dev_err = A->ctx->dev_err;
     cudaLaunchAttribute attr[1];
     const cudaLaunchConfig_t cfg =
@@ -2245,7 +2246,7 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
         HHP_CUDA(cudaStreamSynchronize(st));
     }
     if (dev_err != DEV_OK) {
-        set_error("a bounded device wait timed out inside the SpMV kernel");
+        set_error("a bounded device wait timed out (%s)", ilu ? "ILU(0) level barrier" : "exchange of a one-kernel solve");
         result = HHP_ERR_TIMEOUT;
     }
     if (xt && host) {

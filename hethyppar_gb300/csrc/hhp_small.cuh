@@ -40,7 +40,8 @@ constexpr int kSmallClusterRows = 6144;   // 5-point, 4096 rows: 9.1 against 13.
 // The count starts one below 2^32: a launch of 152 blocks passes 2^32 every 28 million exchanges, and so
 // every launch does in its first.
 constexpr unsigned kSmallCount0 = 0xffffffffu;
-constexpr int kSmallPolls = 1 << 20;      // reads of the count before giving up (~0.5 us each)
+constexpr int kSmallPolls = 1 << 20;      // reads of the count before giving up (~0.5 us each); the
+                                          // variable HHP_SMALL_POLLS sets another limit
 
 struct SmallArgs {
     DevScal *sc;
@@ -60,7 +61,7 @@ struct SmallArgs {
     double *rec;              // 2 sets of kSmallQ * grid partial sums, used in turn
     unsigned *arrived;        // blocks that have arrived, over all exchanges, from kSmallCount0
     double *hist;
-    int hist_cap;
+    int hist_cap, polls;
     int *dev_err;
 };
 
@@ -146,7 +147,7 @@ __device__ __forceinline__ bool exchange(const SmallArgs &a, SmallShared &sh, co
             asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(a.arrived) : "memory");
             const unsigned target = kSmallCount0 + e * static_cast<unsigned>(G);
             bool all = false;
-            for (int i = 0; i < kSmallPolls && !all; ++i) {
+            for (int i = 0; i < a.polls && !all; ++i) {
                 unsigned seen;
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.arrived) : "memory");
                 all = count_reached(seen, target);
