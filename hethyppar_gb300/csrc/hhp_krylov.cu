@@ -2247,6 +2247,8 @@ hhp_status solve_any(hhp_mat *A, const double *b_in, double *x_io, const double 
     }
     if (dev_err != DEV_OK) {
         set_error("a bounded device wait timed out (%s)", ilu ? "ILU(0) level barrier" : "exchange of a one-kernel solve");
+        // reported: the word would make every later launch of the context return without a result
+        HHP_CUDA(cudaMemsetAsync(ctx->dev_err, 0, sizeof(int), st));
         result = HHP_ERR_TIMEOUT;
     }
     if (xt && host) {

@@ -2,6 +2,7 @@
 first exchange. The solve reports it, and the context and the matrix go on."""
 import numpy as np
 import pytest
+import torch
 
 from hethyppar_gb300 import HHPError, Matrix, bicgstab, synth
 from oracle import oracle as orc
@@ -37,3 +38,16 @@ def test_reported_and_over(ctx, monkeypatch, timed_out, precision):
         x, r = bicgstab(ctx, A, s.b, rtol=1e-10, precision=precision)
         d = s.b - orc.spmv(s.rowptr, s.col, s.val, x)
         assert r.status == 0 and np.sqrt(orc.dot(d, d) / orc.dot(s.b, s.b)) <= 1.0000001e-10
+
+
+def test_products_after_it_are_computed(ctx, timed_out):
+    """The error that the solve has reported does not stop what the caller launches next."""
+    s, A, _ = timed_out
+    x = torch.as_tensor(np.random.default_rng(3).standard_normal(s.n)).cuda()
+    y, z = torch.zeros_like(x), torch.zeros_like(x)
+    A.spmv_dev(x, y)
+    A.spmv_t_dev(x, z)
+    torch.cuda.synchronize()
+    assert np.array_equal(y.cpu().numpy(), orc.spmv(s.rowptr, s.col, s.val, x.cpu().numpy(), fma=True))
+    tr, tc, tv = orc.csr_to_csc(s.rowptr, s.col, s.val, s.n)
+    assert np.array_equal(z.cpu().numpy(), orc.spmv(tr, tc, tv, x.cpu().numpy(), fma=True))
