@@ -71,8 +71,10 @@ struct SellHost {
 };
 
 // Builds the plan from a host rowptr: rpl rows per lane (H = 32*rpl rows per slice), rows longer
-// than long_thr go to chunks of at most cap nonzeros, `window` rows per length-sort window.
-void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int window, SellHost &out);
+// than long_thr go to chunks of at most cap nonzeros, `window` rows per length-sort window. Rows that
+// need sorting at rpl take rpl_sorted rows per lane instead (0: rpl), and are sorted if they need it there.
+void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int window, SellHost &out,
+                int rpl_sorted = 0);
 // Deals the plan's units (slices, then chunks) to n_warps warps, balancing their step counts;
 // warp w processes warp_units[warp_ptr[w] .. warp_ptr[w+1]) in ascending order.
 void assign_units(const SellHost &P, int n_warps, std::vector<int> &warp_ptr, std::vector<int> &warp_units,

@@ -55,13 +55,12 @@ void parallel_ranges(size_t n, size_t min_per_thread, Fn fn) {
 
 }  // namespace
 
-void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int window, SellHost &P) {
+void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int window, SellHost &P, int rpl_sorted) {
     P = SellHost();
     P.rpl = rpl;
     P.H = 32 * rpl;
     P.long_thr = long_thr;
     P.cap = cap;
-    const int H = P.H;
     // rows up to long_thr go to slices in row order, longer ones to chunks: counted per range of
     // rows, then placed at each range's offset
     const size_t nr = static_cast<size_t>(m), kRange = 1 << 16;
@@ -113,6 +112,7 @@ void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int wi
     P.long_first.push_back(n_chunks);
     // slice widths of an order (H rows per slice, the longest row sets the width), in parallel
     auto widths = [&](const std::vector<int> &ord, std::vector<int> &w) {
+        const int H = P.H;
         const size_t ns = (ord.size() + static_cast<size_t>(H) - 1) / static_cast<size_t>(H);
         w.assign(ns, 0);
         parallel_ranges(ns, 2048, [&](size_t b, size_t e) {
@@ -129,12 +129,22 @@ void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int wi
     auto padded = [&](const std::vector<int> &ord) {
         widths(ord, width);
         long long tot = 0;
-        for (int x : width) tot += static_cast<long long>(x) * H;
+        for (int x : width) tot += static_cast<long long>(x) * P.H;
         return tot;
     };
-    long long tot = padded(order);
+    auto pads = [&] {  // in natural order, too much
+        const long long tot = padded(order);
+        return short_nnz > 0 && static_cast<double>(tot) > 1.15 * static_cast<double>(short_nnz);
+    };
+    bool sort = pads();
+    if (sort && rpl_sorted > 0 && rpl_sorted != rpl) {
+        P.rpl = rpl_sorted;
+        P.H = 32 * rpl_sorted;
+        sort = pads();
+    }
+    const int H = P.H;
     P.sorted = false;
-    if (short_nnz > 0 && static_cast<double>(tot) > 1.15 * static_cast<double>(short_nnz)) {
+    if (sort) {
         const size_t nwin = (order.size() + static_cast<size_t>(window) - 1) / static_cast<size_t>(window);
         parallel_ranges(nwin, 4, [&](size_t wb, size_t we) {
             for (size_t wi = wb; wi < we; ++wi) {
@@ -146,7 +156,7 @@ void build_plan(int m, const int *rowptr, int rpl, int long_thr, int cap, int wi
                 });
             }
         });
-        tot = padded(order);
+        padded(order);
         P.sorted = true;
     }
     P.has_perm = P.sorted || !P.long_rows.empty();

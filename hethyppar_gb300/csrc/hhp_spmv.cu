@@ -913,16 +913,14 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
         R = t.rpl32 == 2 ? 2 : 4;
         U = t.spmv_unroll == 2 || t.spmv_unroll == 4 ? t.spmv_unroll : 4;
         cps = t.ctas_per_sm > 0 ? t.ctas_per_sm : 3;
-        build_plan(A->m, A->rowptr_host.data(), R, std::max(t.long_thr, 1), std::max(t.cap, 32),
-                   std::max(t.window, 1), h);
         // length-sorted rows: 2 per lane on 4 CTAs, shorter chains in the slices of long rows and more
         // warps for the gathers (power law, back to back: 40k rows 35 -> 25 us, 300k 62 -> 45, 3.5M 153
         // -> 137)
-        if (h.sorted && R == 4 && t.rpl32 != 2) {
-            R = 2;
+        build_plan(A->m, A->rowptr_host.data(), R, std::max(t.long_thr, 1), std::max(t.cap, 32),
+                   std::max(t.window, 1), h, 2);
+        if (h.rpl != R) {
+            R = h.rpl;
             if (t.ctas_per_sm <= 0) cps = 4;
-            build_plan(A->m, A->rowptr_host.data(), R, std::max(t.long_thr, 1), std::max(t.cap, 32),
-                       std::max(t.window, 1), h);
         }
     }
     // Uniform diagonals (stencils): every entry on one of at most kMaxDiag diagonals, rows in
