@@ -941,7 +941,8 @@ hhp_status build_plan_dev(hhp_mat *A, PlanDev &p) {
         HHP_CUDA(cudaMemcpy(hc.data(), A->col, sizeof(int) * n_pre, cudaMemcpyDeviceToHost));
         // FP32: the prefix may hold any number of absent entries, as the first rows of a grid lie on its
         // boundary (11,000 rows of a 100^3 grid are its first plane and a tenth, 13 % padding; the mixed
-        // solve 44.2 -> 38.6 us an iteration). FP64 leaves such grids to 16-bit offsets, with which
+        // solve 44.2 -> 38.6 us an iteration, for a check of all columns: matrix and first FP32 product 4.9 ->
+        // 7.7 ms, paid back within 500 iterations). FP64 leaves such grids to 16-bit offsets, with which
         // their solves are faster (100^3: 77.1 against 79.1 us an iteration).
         const double pad = std::is_same<VT, double>::value ? 0.10 : 1e9;
         if (uniform_diagonals(m_pre, rp.data(), hc.data(), kMaxDiag, pad, doff, K, mask)) {
