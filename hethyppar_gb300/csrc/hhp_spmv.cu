@@ -757,24 +757,26 @@ cudaError_t launch_ru(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaSt
     return p.d16 ? launch_rud<VT, R, U, true>(ep, p, a, s) : launch_rud<VT, R, U, false>(ep, p, a, s);
 }
 
-// FP64 products of 7 uniform diagonals in the solve loop, with stream and vectors between kStreamKeep and
-// kStreamFar, take the general kernel (the same bits). Half of what the loop touches then still survives
-// in the L2 from one product to the next, and it survives best under the general kernel's slower, evener
-// stream; us a merged iteration, general / k_spmv_uni: 600x40x40 75.3 / 78.1, 107^3 90.7 / 92.0, 112^3
-// 100.3 / 101.6; outside, 500x40x40 68.2 / 67.1, 118^3 116.2 / 115.4, 160^3 248 / 244.
+// FP64 products of 7 uniform diagonals take the general kernel (the same bits) where what lies between two uses
+// of a word is between kStreamKeep and kStreamFar: the stream and the loop's 8 vectors in the solve loop, the
+// stream, x and y of plain products one after another. Part of it then still survives in the L2 from one
+// product to the next, and it survives best under the general kernel's slower, evener stream; us a merged
+// iteration, general / k_spmv_uni: 600x40x40 75.3 / 78.1, 107^3 90.7 / 92.0, 112^3 100.3 / 101.6; outside,
+// 500x40x40 68.2 / 67.1, 118^3 116.2 / 115.4, 160^3 248 / 244. A plain product: 120^3 29.3 / 30.0, 128^3 34.0 /
+// 35.1 (with alpha and beta 35.7 / 37.5, 41.9 / 43.5); outside, 112^3 25.2 / 23.6, 160^3 62.0 / 59.6.
 constexpr long long kStreamFar = 180LL << 20;
 template <typename VT>
-bool general_loop(EpKind ep, const PlanDev &p, const SellArgs<VT> &a) {
-    const long long bytes = (p.total + 8LL * a.m) * static_cast<long long>(sizeof(VT));
-    return std::is_same<VT, double>::value && p.K == 7 && (ep == EP_DOT1 || ep == EP_DOT2 || ep == EP_DOT3) &&
-           bytes > kStreamKeep && bytes < kStreamFar;
+bool general_uni(EpKind ep, const PlanDev &p, const SellArgs<VT> &a) {
+    const bool loop = ep == EP_DOT1 || ep == EP_DOT2 || ep == EP_DOT3;
+    const long long bytes = (p.total + (loop ? 8LL : 2LL) * a.m) * static_cast<long long>(sizeof(VT));
+    return std::is_same<VT, double>::value && p.K == 7 && bytes > kStreamKeep && bytes < kStreamFar;
 }
 
 // Rows per lane come from the plan, the unroll from the tuning (2 or 4 steps in flight per lane).
 template <typename VT>
 cudaError_t launch_ep(EpKind ep, const PlanDev &p, const SellArgs<VT> &a, cudaStream_t s) {
     const bool u2 = p.unroll == 2;
-    if (p.mask8 && !general_loop<VT>(ep, p, a)) {  // 5 or 7 uniform diagonals in the default row layout
+    if (p.mask8 && !general_uni<VT>(ep, p, a)) {  // 5 or 7 uniform diagonals in the default row layout
         if constexpr (std::is_same<VT, double>::value)
             return p.K == 5 ? launch_uni<VT, 2, 5, 5>(ep, p, a, s) : launch_uni<VT, 2, 7, 5>(ep, p, a, s);
         else

@@ -134,3 +134,21 @@ def test_loop_kernel_by_size(ctx, dims):
         x, r = bicgstab(ctx, A, b, rtol=1e-12, maxit=3, loop=loop)
         assert r.iters == 3 and np.max(np.abs(x - ref)) <= 1e-10 * max(1.0, np.max(np.abs(ref)))
     A.close()
+
+
+@pytest.mark.parametrize("dims", [(580, 50, 50), (590, 50, 50), (1040, 50, 50), (1055, 50, 50)])
+def test_product_kernel_by_size(ctx, dims):
+    """Plain products on both sides of the sizes that take the general kernel: row sums bit for bit."""
+    rp, col, val = synth._stencil(dims, 20.0, (1.0, 0.5, 0.25))
+    n = rp.size - 1
+    rng = np.random.default_rng(n)
+    x, y0 = rng.standard_normal(n), rng.standard_normal(n)
+    A = Matrix.from_csr(ctx, rp, col, val)
+    want = orc.spmv(rp, col, val, x, fma=True)
+    xd, y = dev(x), torch.empty(n, dtype=torch.float64, device="cuda")
+    A.spmv_dev(xd, y)
+    assert np.array_equal(y.cpu().numpy(), want)
+    y = dev(y0)
+    A.spmv_dev(xd, y, 0.5, 1.0)  # exact up to the one rounding of the sum
+    assert np.array_equal(y.cpu().numpy(), 0.5 * want + y0)
+    A.close()
