@@ -1434,8 +1434,8 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
     const int *stop = &sc->status;
     hhp_status st = HHP_OK;
     auto kp = [&](cudaStream_t q, cudaGraphConditionalHandle c, int first_in_body) -> hhp_status {
-        HHP_CUDA(launch_k(k_p<T>, dim3(s->nblk), dim3(fp32 ? s->nthr_u32 : s->nthr_u64), 0, q, sc, P, V, R, nu, part_xr, part_s, s->nblk,
-                          s->hist, s->hist_cap, c, first_in_body, A->ctx->dev_err, 1,
+        HHP_CUDA(launch_k(k_p<T>, dim3(s->nblk), dim3(fp32 ? s->nthr_u32 : s->nthr_u64), 0, q, sc, P, V, R, nu, part_xr,
+                          part_s, s->nblk, s->hist, s->hist_cap, c, first_in_body, A->ctx->dev_err, 1,
                           static_cast<const int *>(nullptr)));
         return HHP_OK;
     };
@@ -1497,9 +1497,9 @@ hhp_status capture_loop(Solver *s, cudaStream_t stream, DevScal *sc, T *X, T *R,
             st = launch_spmv32(A, s->s2, EP_DOT3, S, Tv, S, stop, R0);
             if (st != HHP_OK) break;
             if (launch_k(s->narrow32 ? k_xrp_ru<kNarrow> : k_xrp_ru<512>, dim3(s->nblk),
-                         dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, s->s2, s->sc32, s->X, s->D32, s->R32, s->P32,
-                         s->S32, s->T32, s->V32, nu4, parts_of(pl), part_s, s->nblk, s->hist, s->hist_cap, cond,
-                         icond_body, k == 0 ? 1 : 0, A->ctx->dev_err, 1) != cudaSuccess) {
+                         dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, s->s2, s->sc32,
+                         s->X, s->D32, s->R32, s->P32, s->S32, s->T32, s->V32, nu4, parts_of(pl), part_s, s->nblk, s->hist,
+                         s->hist_cap, cond, icond_body, k == 0 ? 1 : 0, A->ctx->dev_err, 1) != cudaSuccess) {
                 st = HHP_ERR_CUDA;
                 break;
             }
@@ -1623,16 +1623,18 @@ SmallKernel small_kernel(bool merged, bool cluster, bool mix) {
                   : (cluster ? k_small<false, true> : k_small<false, false>);
 }
 
-// Decides once per matrix whether its loop runs as k_small (FP64) and k_small_mix, and lays out what that needs: at most
-// kSmallRows rows, none of them cut into chunks (a row is one thread's), of at most kSmallMaxK entries,
-// and the blocks' entries in shared memory. The gain over the graph loop falls with
-// the size (5-point stencils: 1.9x at 8,100 rows, 1.7x at 16,384, 1.34x at 62,500), as the FP64 work per
-// SM grows; the line lies where it is about 1.5x, so that the loop of a system of tens of thousands of
-// rows and more keeps its summation order and its 4 or 5 launches an iteration.
+// Decides once per matrix whether its loop runs as k_small (FP64) and k_small_mix, and lays out what that
+// needs: at most kSmallRows rows, none of them cut into chunks (a row is one thread's), of at most kSmallMaxK
+// entries, and the blocks' entries in shared memory. The gain over the graph loop falls with the size
+// (5-point stencils: 1.9x at 8,100 rows, 1.7x at 16,384, 1.34x at 62,500), as the FP64 work per SM grows.
+// The line is not where the gain ends but where it was still 1.5x: larger systems keep the summation order
+// that they had, and the schedules "merged" and "classic" their 4 and 5 launches an iteration there, which
+// callers count (hhp_ctx_kernel_launches; a test does at 65,536 rows).
 constexpr int kSmallRows = 40000;
-// The mixed form's line: its counts, and with them the solution within its tolerance, move more with the
-// order of the sums (2D stencils at rtol 1e-12: by 3e-10 up to 125^2, by 1e-9 at 200^2, as two runs of the
-// graph loop with other sums would), so larger systems keep the loop they had.
+// The mixed form's line, again not where the gain ends (1.9x at 40,000 rows): its counts, and with them the
+// solution within its tolerance, move more with the order of the sums (2D stencils at rtol 1e-12: by 3e-10 up
+// to 125^2, by 1e-9 at 200^2, as two runs of the graph loop with other sums would), so larger systems keep the
+// loop they had.
 constexpr int kSmallMixRows = 16384;
 bool small_mix(const Solver *s) { return s->small_grid > 0 && s->n <= kSmallMixRows; }
 
@@ -1987,8 +1989,8 @@ hhp_status run_direct_mix(Solver *s, bool merged) {
                                   s->V32, s->R0_32, nu4, parts_of(pl), s->part_s32));
                 HHP_TRY(launch_spmv32(A, st, EP_DOT3, s->S32, s->T32, s->S32, stop, s->R0_32));
                 HHP_CUDA(launch_k(s->narrow32 ? k_xrp_ru<kNarrow> : k_xrp_ru<512>, dim3(s->nblk),
-                         dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, st, s->sc32, s->X, s->D32, s->R32,
-                                  s->P32, s->S32, s->T32, s->V32, nu4, parts_of(pl), s->part_s32, s->nblk, s->hist,
+                                  dim3(s->narrow32 ? std::min(s->nthr_u32, kNarrow) : s->nthr_u32), 0, st, s->sc32,
+                                  s->X, s->D32, s->R32, s->P32, s->S32, s->T32, s->V32, nu4, parts_of(pl), s->part_s32, s->nblk, s->hist,
                                   s->hist_cap, none, none, k == 0 ? 1 : 0, A->ctx->dev_err, 0));
             } else {
                 HHP_CUDA(launch_k(k_s<float>, dim3(s->nblk), dim3(s->nthr), 0, st, s->sc32, s->S32, s->R32, s->V32,

