@@ -292,34 +292,51 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) k_mp_spmv(int m, int nnz
     }
 }
 
-// Adds each row's carries to its y, once: the warp of the first CTA carrying the row sums the run (CTAs
-// c, c + 1, ... with that row, as the rows ascend), strided over the lanes and then across them, in an order
-// that the run's length alone decides. Four carries of a lane are requested at once: a thread that walked
-// the run alone waited for each (one row of 777,777 entries over 760 CTAs: 106.7 us a call, so 12.4).
+// Adds each row's carries to its y, once: the first CTA carrying a row stands for its run (CTAs c, c + 1, ...
+// with that row, as the rows ascend). A run of up to kRun carries, as between even tiles, is its thread's: all
+// requested at once, added in CTA order. A longer one is its warp's: strided over the lanes, four requests each,
+// then added across them, in an order that the run's length alone decides. (A thread that walked a long run
+// alone waited for each carry: one row of 777,777 entries over 760 CTAs 106.7 us a call, so 12.4. A warp for every
+// carry cost rows of 17 entries 0.5 us of 45.)
+constexpr int kRun = 4;
 __global__ void k_mp_fixup(int n_cta, double alpha, double *y, const double *carry_val, const int *carry_row) {
-    constexpr int N = 4;
-    const int c = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the first kernel's stores are complete and visible
-    if (c >= n_cta) return;
-    const int row = carry_row[c];
-    if (row < 0 || (c > 0 && carry_row[c - 1] == row)) return;
-    double s = 0.0;
-    for (int q = c + lane;; q += 32 * N) {
-        int r[N];
-        double v[N];
+    auto row_of = [&](int q) { return q >= 0 && q < n_cta ? carry_row[q] : -1; };
+    const int row = row_of(c), before = row_of(c - 1);
+    int next[kRun];
+    double v[kRun];
 #pragma unroll
-        for (int u = 0; u < N; ++u) {
-            const bool in = q + 32 * u < n_cta;
-            r[u] = in ? carry_row[q + 32 * u] : -1;
-            v[u] = in ? carry_val[q + 32 * u] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < N; ++u)
-            if (r[u] == row) s += v[u];
-        if (r[N - 1] != row) break;
+    for (int u = 0; u < kRun; ++u) {
+        next[u] = row_of(c + u + 1);
+        v[u] = c + u < n_cta ? carry_val[c + u] : 0.0;
     }
-    s = hhp::warp_sum(s);
-    if (lane == 0) y[row] = fma(alpha, s, y[row]);
+    const bool first = row >= 0 && before != row, far = first && next[kRun - 1] == row;
+    if (first && !far) {
+        double s = v[0];
+#pragma unroll
+        for (int u = 1; u < kRun; ++u)
+            if (next[u - 1] == row) s += v[u];
+        y[row] = fma(alpha, s, y[row]);
+    }
+    for (unsigned left = __ballot_sync(0xffffffffu, far); left != 0; left &= left - 1) {
+        const int src = __ffs(left) - 1, r = __shfl_sync(0xffffffffu, row, src);
+        double s = 0.0;
+        for (int q = c + src;; q += 32 * kRun) {  // this lane's: the run's first carry + lane, ...
+            bool on[kRun];
+#pragma unroll
+            for (int u = 0; u < kRun; ++u) {
+                on[u] = row_of(q + 32 * u) == r;
+                v[u] = on[u] ? carry_val[q + 32 * u] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < kRun; ++u)
+                if (on[u]) s += v[u];
+            if (!on[kRun - 1]) break;
+        }
+        s = hhp::warp_sum(s);
+        if (lane == 0) y[r] = fma(alpha, s, y[r]);
+    }
 }
 
 hhp_status scratch_for_current_device(Scratch &out) {
@@ -375,7 +392,7 @@ extern "C" hhp_status hhp_spmv_csr_noalloc(int m, int n, int nnz, const int *row
     // last block has ended, not a launch later (450k banded rows 46.8 -> 45.1 us a call, one row of 100,000 entries
     // 10.3 -> 8.3)
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>((n_cta + 7) / 8));  // a warp per carry
+    cfg.gridDim = dim3(static_cast<unsigned>((n_cta + 255) / 256));
     cfg.blockDim = dim3(256);
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
