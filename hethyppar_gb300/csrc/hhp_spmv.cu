@@ -586,7 +586,7 @@ __device__ __forceinline__ void load_run(VT (&o)[N], const VT *x, int i, int off
 
 // The value stream's words in k_spmv_uni. ONCE (streaming loads, first out of the caches): in the solve
 // loop's products where the stream and the loop's vectors together do not fit the L2 (kStreamKeep); the
-// vectors then stay there between its kernels. 160^3 mixed: DRAM reads of K_S 33 -> 11 MB, of
+// vectors then stay there between its kernels. 160^3 mixed: DRAM reads of K_S 33 -> 14 MB, of
 // K_XRP_RU 74 -> 44 MB, an inner iteration 109.2 -> 103.7 us; 140^3 79.0 -> 72.8, 125^3 58.9 -> 57.0; FP64
 // 1024^2 73.8 -> 72.9. Where all fits it costs 3 % (100^3 mixed, 60 MB: 38.6 -> 39.9), and a plain product
 // has no vectors to keep. (An evict-first policy operand did the same in FP32, less well: 105.2; the

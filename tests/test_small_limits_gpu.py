@@ -48,9 +48,8 @@ def test_two_systems_in_turn(ctx, monkeypatch, pair, graph):
     B.close()
 
 
-@pytest.mark.parametrize("pair", PAIRS)
-def test_two_contexts_on_two_threads(pair):
-    systems = _systems(pair)
+def _together(systems):
+    """Every call for each of the systems, a context and a thread each."""
     failed = []
 
     def work(system):
@@ -69,3 +68,14 @@ def test_two_contexts_on_two_threads(pair):
     for t in threads:
         t.join()
     assert not failed, failed
+
+
+@pytest.mark.parametrize("pair", PAIRS)
+def test_two_contexts_on_two_threads(pair):
+    _together(_systems(pair))
+
+
+def test_two_grids_that_do_not_fit_together():
+    """One block of either takes more than half of an SM's shared memory: one solve's grid waits for the other's."""
+    m, width = 20_000, 62
+    _together([(*_dominant(m, width, seed), np.random.default_rng(seed).standard_normal(m)) for seed in (1, 2)])
